@@ -307,3 +307,70 @@ def tolerance(case):
 # are 4.9e-4, 3.9e-3 and 8.4e-7; "max" leaves room for a query or key element, rounded to the other
 # side by another order of the norm's sum, in a short sequence.
 TOL = {"f16": {"rel": 1e-3, "max": 4e-3}, "bf16": {"rel": 7e-3, "max": 3e-2}, "f32": {"rel": 1e-6, "max": 1e-5}}
+
+
+def _exact_append(s, q, k, v, pos, kp, vp, slots):
+    """The step's rows normalised, rotated and stored in 64 bits: q [n, heads, D]; kp and vp
+    [slots, heads, D] take the new rows.  The sin / cos tables are inputs as they stand."""
+    def rotated(x, heads, w):
+        x = x.double().view(-1, heads, D)
+        if s["case"]["norm"]:
+            x = w.double() * x / torch.sqrt((x * x).mean(-1, keepdim=True) + EPS)
+        at = pos.long()
+        sin, cos = (t.view(-1, D)[at, ::2].double().unsqueeze(1) for t in (s["sin"], s["cos"]))
+        lo, hi = x[..., :D // 2], x[..., D // 2:]
+        return torch.cat([lo * cos - hi * sin, lo * sin + hi * cos], -1)
+    kp[slots] = rotated(k, s["case"]["kv"], s["norms"][1])
+    vp[slots] = v.double().view(-1, s["case"]["kv"], D)
+    return rotated(q, s["case"]["q"], s["norms"][0])
+
+
+def _exact_attention(q, k, v, start, kv, dtype):
+    """q [n, heads, D] at positions start.. over k and v [tokens, kv, D]; q and k enter rounded to
+    the type that the path holds them in."""
+    n, heads = q.shape[:2]
+    q, k = (x.to(dtype).double() for x in (q, k))
+    hidden = torch.arange(len(k), device="cuda") > start + torch.arange(n, device="cuda").unsqueeze(1)
+    out = []
+    for h, group in enumerate(q.transpose(0, 1).chunk(kv)):  # the query heads of KV head h
+        scores = (group @ k[:, h].T / math.sqrt(D)).masked_fill_(hidden, -math.inf)
+        out.append(torch.softmax(scores, -1) @ v[:, h])
+    return torch.cat(out).transpose(0, 1).reshape(n, heads * D)
+
+
+def exact(case, seed):
+    """What run returns, in 64 bits; a fork's outputs are bytes."""
+    if case["kind"] == "fork":
+        return None
+    s = prepare(dict(case, call="eager") if case["kind"] == "decode" else case, seed)
+    s["qk"].copy_(s["fresh"])
+    kv, dtype, out = case["kv"], DTYPES[case["dtype"]], torch.zeros_like(s["out"], dtype=torch.float64)
+    paged = case.get("layout") != "contiguous"
+    # pools as [layer, slot, head, D]
+    kps, vps = (t.double().view(-1, t.shape[-4], kv, BS, D).transpose(2, 3).reshape(-1, t.shape[-4] * BS, kv, D) if paged
+                else t.double().view(t.shape[0], -1, kv, D) for t in (s["kp"], s["vp"]))
+
+    def keys(table_row, n):
+        at = torch.arange(n, device="cuda")
+        return at if table_row is None else table_row[at // BS].long() * BS + at % BS
+    if case["kind"] == "decode":
+        for i in range(case["layers"]):
+            q = _exact_append(s, s["q"][i], s["k"][i], s["v"][i], s["pos"], kps[i], vps[i], s["slots"])
+            for b, n in enumerate(s["pos"].tolist()):
+                at = keys(s["table"][b] if paged else None, n + 1)
+                out[i, b] = _exact_attention(q[b:b + 1], kps[i][at], vps[i][at], n, kv, dtype)[0]
+    else:
+        row = 0
+        for st in s["steps"]:
+            q = _exact_append(s, st["q"], st["k"], st["v"], st["pos"], kps[0], vps[0], st["slots"])
+            for r, start in enumerate(st["start"].tolist()):
+                a, b = st["cu"][r:r + 2].tolist()
+                at = keys(st["table"][r], start + b - a)
+                out[row + a:row + b] = _exact_attention(q[a:b], kps[0][at], vps[0][at], start, kv, dtype)
+            row += st["n"]
+
+    def stored(pools, like):
+        if paged:
+            pools = pools.view(len(pools), -1, BS, kv, D).transpose(2, 3)
+        return pools.reshape(like.shape)
+    return dict(out=out, k=stored(kps, s["kp"]), v=stored(vps, s["vp"]))
