@@ -151,10 +151,10 @@ KPX_API int kpx_paged_decode(void* out, const void* q, const void* k_pool, const
 
 /* kpx_paged_decode for launches that the caller overlaps on the GPU with other launches of
  * this library (consecutive layers or requests on different streams, each launch with ITS OWN
- * workspace).  Same arguments and results.  The kernel then runs as three CTAs of four warps per
- * SM instead of one CTA of twelve, so that an SM passes from one launch to the next a third at
- * a time while the earlier launch's last warps finish; run alone, kpx_paged_decode's single
- * large CTA is the faster form.  No reference counterpart (the reference runs one kernel at a
+ * workspace).  Same arguments and results.  The kernel then runs as several small CTAs per SM
+ * (16-bit caches: two of four warps; fp32: three of two) instead of one large one, so that an SM
+ * passes from one launch to the next piece by piece while the earlier launch's last warps finish;
+ * run alone, kpx_paged_decode's single large CTA is the faster form.  No reference counterpart (the reference runs one kernel at a
  * time on one stream). */
 KPX_API int kpx_paged_decode_overlapped(void* out, const void* q, const void* k_pool, const void* v_pool,
                                         const kpx_kv_layout* layout, const int32_t* block_table,
@@ -199,8 +199,8 @@ KPX_API int kpx_paged_decode_planned(void* out, const void* q, const void* k_poo
  * it writes.  Each (sequence, kv head) row pair is stored by the warp that finishes that
  * sequence's last cached block.  Workspace, status word and capture rules as kpx_paged_decode.
  * flags: KPX_DECODE_OVERLAPPED when the caller runs this launch concurrently with other launches
- * of this library (another stream, ANOTHER workspace): the kernel then uses three small CTAs per
- * SM so that SMs pass from one launch to the next in thirds; 0 otherwise.
+ * of this library (another stream, ANOTHER workspace): the kernel then uses small CTAs, as
+ * kpx_paged_decode_overlapped does; 0 otherwise.
  * Replaces the decode-step sequence RoPEGpuPosLayer -> KVCacheLayer(K), KVCacheLayer(V) ->
  * FlashAttentionDecodeLayer / MHAGpuPosLayer of attention_qkv_with_graph and
  * attention_mha_with_graph (kuiper/source/model/qwen3.cpp:1052-1127,

@@ -176,13 +176,13 @@ extern "C" int kpx_decode_plan(void* plan, int64_t plan_bytes, const kpx_kv_layo
   p.num_q_heads = num_q_heads;
   p.num_kv_heads = layout->num_kv_heads;
   p.kv_mul = num_q_heads / layout->num_kv_heads;
-  const int qh = heads_per_warp(p.kv_mul);
+  const int qh = layout->dtype == KPX_F32 ? heads_per_warp(p.kv_mul) : kMmaHeads;
   p.head_groups = (p.kv_mul + qh - 1) / qh;
-  // the warps of the launch forms that take a plan: 12 per SM for 16-bit caches (one CTA of 12
-  // or three of 4), 6 for fp32
+  // the warps of the launch forms that take a plan: 8 per SM for 16-bit caches (one CTA of 8
+  // or two of 4), 6 for fp32
   int sms = device_info().sm_count;
   if (sms > kMaxSms) sms = kMaxSms;
-  const int workers = sms * (layout->dtype == KPX_F32 ? 6 : 12);
+  const int workers = sms * (layout->dtype == KPX_F32 ? 6 : kMmaWarpsPerSm);
   decode_plan_kernel<<<(workers + kPlanThreads - 1) / kPlanThreads, kPlanThreads, 0, s>>>(
       p, static_cast<int32_t*>(plan), workers);
   return cuda_status(cudaGetLastError());
@@ -257,6 +257,10 @@ int kpx::decode_rows(void* out, const void* q, const void* k_pool, const void* v
   p.counters = reinterpret_cast<int32_t*>(static_cast<uint8_t*>(workspace) + kStatusBytes);
   p.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + kStatusBytes +
                                         counter_bytes(num_q_heads, layout->num_kv_heads));
+  p.group_counters = reinterpret_cast<int32_t*>(
+      p.partials + int64_t(kMinPartialSlots - 1) * slot_floats_of(heads_per_warp(num_q_heads / layout->num_kv_heads)));
+  p.small = 0;
+  p.slot_heads = 0;
   p.block_stride_b = layout->block_stride * eb;
   p.head_stride_b = layout->head_stride * eb;
   p.token_stride_b = layout->token_stride * eb;

@@ -1,9 +1,10 @@
 // Paged GQA decode attention for sm_100a: warp-granular split-KV streaming + merge.
 //
-// This header holds the kernel, its launch forms and the per-element-type dispatcher.  It is
-// included by kpx_decode.cu (entry points) and by one translation unit per element type
-// (kpx_decode_f16.cu, _bf16.cu, _f32.cu), each of which instantiates dispatch_decode<T> once, so
-// that the three sets of kernels compile side by side.
+// This header holds what all decode kernels share (parameters, the plan of a step, the walk along
+// the line of blocks) and the kernel for fp32 caches with its launch forms; the kernel for 16-bit
+// caches is in kpx_decode_mma.cuh.  It is included by kpx_decode.cu (entry points) and by one
+// translation unit per element type (kpx_decode_f16.cu, _bf16.cu, _f32.cu), each of which defines
+// dispatch_decode<T> once, so that the three sets of kernels compile side by side.
 //
 // Work decomposition.  The cache of sequence b holds len_b tokens in blocks of 16.
 // An "item" is one (sequence, kv head, query-head group) triple; its work is the
@@ -42,6 +43,7 @@ constexpr int kD = 128;          // head size
 constexpr int kBS = 16;          // tokens per block
 constexpr int kMaxBatch = 512;   // sequences per launch (their block prefix lives in smem)
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int kMmaHeads = 8, kMmaWarpsPerSm = 8;  // 16-bit caches: query heads per warp, warps per SM
 
 struct DecodeParams {
   void* out;
@@ -80,6 +82,10 @@ struct DecodeParams {
   // A plan of this step (nullptr: none), see the layout below: what every launch of the step
   // would otherwise work out again in its prologue.
   const int32_t* plan;
+  // 16-bit caches (kpx_decode_mma.cuh): few blocks per warp; heads a workspace slot holds; counters
+  // of the two-level assembly.
+  int32_t small, slot_heads;
+  int32_t* group_counters;
 };
 
 // Plan of one decode step.  The launches of a step (one per layer) all see the same lengths and
@@ -149,6 +155,40 @@ __device__ __forceinline__ void block_prefix(const DecodeParams& p, int* prefix,
     }
   }
   __syncthreads();
+}
+
+// A sequence without tokens gets zeros (no warp ever visits it); CTAs share the rows.
+// In the fused step its only token is the new one: every head's output is that token's V
+// row, and its rotated K (position 0: unchanged) and V rows go to slot 0 of its first block.
+template <typename T, bool kFused>
+__device__ __forceinline__ void write_empty_rows(const DecodeParams& p, const int* prefix, int tid, int nthreads) {
+  for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
+    if (prefix[b + 1] != prefix[b]) continue;
+    T* o = static_cast<T*>(p.out) + int64_t(b) * p.num_q_heads * kD;
+    if (!kFused) {
+      for (int e = tid; e < p.num_q_heads * kD; e += nthreads) o[e] = Elt<T>::from_float(0.f);
+      continue;
+    }
+    const T* vn = static_cast<const T*>(p.v_new) + int64_t(b) * p.num_kv_heads * kD;
+    for (int e = tid; e < p.num_q_heads * kD; e += nthreads) o[e] = vn[(e / kD / p.kv_mul) * kD + e % kD];
+    const int32_t* row = p.block_table ? p.block_table + int64_t(p.row_index ? p.row_index[b] : b) * p.max_blocks_per_seq : nullptr;
+    int id = row ? row[0] : 0;
+    if (id < 0 || (p.num_blocks > 0 && id >= p.num_blocks)) {
+      if (tid == 0) atomicMax(p.status, KPX_ERR_INVALID_ARGUMENT);
+      continue;
+    }
+    const T* kn = static_cast<const T*>(p.k_new) + int64_t(b) * p.num_kv_heads * kD;
+    for (int e = tid; e < p.num_kv_heads * kD; e += nthreads) {
+      const int h = e / kD, d = e % kD, j = d & (kD / 2 - 1);
+      const float lo = Elt<T>::to_float(kn[h * kD + j]), hi = Elt<T>::to_float(kn[h * kD + kD / 2 + j]);
+      const float sn = __ldg(p.sin_cache + 2 * j), cs = __ldg(p.cos_cache + 2 * j);
+      const float r = d >= kD / 2 ? __fadd_rn(__fmul_rn(lo, sn), __fmul_rn(hi, cs))
+                                  : __fsub_rn(__fmul_rn(lo, cs), __fmul_rn(hi, sn));
+      const int64_t off = int64_t(id) * p.block_stride_b + int64_t(h) * p.head_stride_b + int64_t(d) * int(sizeof(T));
+      *reinterpret_cast<T*>(p.k_pool_w + off) = Elt<T>::from_float(r);
+      *reinterpret_cast<T*>(p.v_pool_w + off) = vn[e];
+    }
+  }
 }
 
 // Position on the line of blocks: sequence b, sub-item (= kv_head*head_groups +
@@ -235,7 +275,8 @@ __device__ __forceinline__ void fence_proxy_async() {
 // pairs (j, j + 64), sin/cos read at pos*128 + 2j, products rounded separately and one rounding
 // to T: the bits rope_append_kernel stores.  Kept out of line so that the streaming loop's
 // register allocation is that of the plain kernel; the caller brackets it with __syncwarp().
-template <typename T, int QH>
+// Rows of the staging area are kRowStride bytes apart.
+template <typename T, int QH, int kRowStride>
 __device__ __noinline__ void stage_new_token(const T* q_kv_group, int hg, int kv_mul, const T* k_row,
                                              const uint8_t* v_row, bool with_kv, const float* sin_row,
                                              const float* cos_row, const int32_t* table_entry,
@@ -259,16 +300,16 @@ __device__ __noinline__ void stage_new_token(const T* q_kv_group, int hg, int kv
       lo_out[e] = Elt<T>::from_float(__fsub_rn(__fmul_rn(lo[e], cs), __fmul_rn(hi[e], sn)));
       hi_out[e] = Elt<T>::from_float(__fadd_rn(__fmul_rn(lo[e], sn), __fmul_rn(hi[e], cs)));
     }
-    uint8_t* dst = stage + r * kRowB;
+    uint8_t* dst = stage + r * kRowStride;
     *reinterpret_cast<uint4*>(dst + g * 16) = *reinterpret_cast<const uint4*>(lo_out);
     *reinterpret_cast<uint4*>(dst + kRowB / 2 + g * 16) = *reinterpret_cast<const uint4*>(hi_out);
   }
   if (with_kv) {
     for (int task = lane; task < kRowB / 16; task += 32)
-      *reinterpret_cast<uint4*>(stage + (QH + 1) * kRowB + task * 16) =
+      *reinterpret_cast<uint4*>(stage + (QH + 1) * kRowStride + task * 16) =
           __ldg(reinterpret_cast<const uint4*>(v_row) + task);
     if (lane == 0)
-      *reinterpret_cast<int32_t*>(stage + (QH + 2) * kRowB) = table_entry ? __ldg(table_entry) : identity_id;
+      *reinterpret_cast<int32_t*>(stage + (QH + 2) * kRowStride) = table_entry ? __ldg(table_entry) : identity_id;
   }
 }
 
@@ -323,36 +364,7 @@ paged_decode_kernel(const DecodeParams p) {
     }
   }
   if (!planned) block_prefix(p, prefix, tid, C::kThreads, warp, lane, blockIdx.x == 0);
-  // a sequence without tokens gets zeros (no warp ever visits it); CTAs share the rows.
-  // In the fused step its only token is the new one: every head's output is that token's V
-  // row, and its rotated K (position 0: unchanged) and V rows go to slot 0 of its first block.
-  for (int b = blockIdx.x; b < p.batch; b += gridDim.x) {
-    if (prefix[b + 1] != prefix[b]) continue;
-    T* o = static_cast<T*>(p.out) + int64_t(b) * p.num_q_heads * kD;
-    if (!kFused) {
-      for (int e = tid; e < p.num_q_heads * kD; e += C::kThreads) o[e] = Elt<T>::from_float(0.f);
-      continue;
-    }
-    const T* vn = static_cast<const T*>(p.v_new) + int64_t(b) * p.num_kv_heads * kD;
-    for (int e = tid; e < p.num_q_heads * kD; e += C::kThreads) o[e] = vn[(e / kD / p.kv_mul) * kD + e % kD];
-    const int32_t* row = p.block_table ? p.block_table + int64_t(p.row_index ? p.row_index[b] : b) * p.max_blocks_per_seq : nullptr;
-    int id = row ? row[0] : 0;
-    if (id < 0 || (p.num_blocks > 0 && id >= p.num_blocks)) {
-      if (tid == 0) atomicMax(p.status, KPX_ERR_INVALID_ARGUMENT);
-      continue;
-    }
-    const T* kn = static_cast<const T*>(p.k_new) + int64_t(b) * p.num_kv_heads * kD;
-    for (int e = tid; e < p.num_kv_heads * kD; e += C::kThreads) {
-      const int h = e / kD, d = e % kD, j = d & (kD / 2 - 1);
-      const float lo = Elt<T>::to_float(kn[h * kD + j]), hi = Elt<T>::to_float(kn[h * kD + kD / 2 + j]);
-      const float sn = __ldg(p.sin_cache + 2 * j), cs = __ldg(p.cos_cache + 2 * j);
-      const float r = d >= kD / 2 ? __fadd_rn(__fmul_rn(lo, sn), __fmul_rn(hi, cs))
-                                  : __fsub_rn(__fmul_rn(lo, cs), __fmul_rn(hi, sn));
-      const int64_t off = int64_t(id) * p.block_stride_b + int64_t(h) * p.head_stride_b + int64_t(d) * C::kEltB;
-      *reinterpret_cast<T*>(p.k_pool_w + off) = Elt<T>::from_float(r);
-      *reinterpret_cast<T*>(p.v_pool_w + off) = vn[e];
-    }
-  }
+  write_empty_rows<T, kFused>(p, prefix, tid, C::kThreads);
   const int64_t total = int64_t(prefix[p.batch]) * p.num_kv_heads * p.head_groups;
   int64_t W_ = int64_t(gridDim.x) * C::kWarps;
   int64_t worker_ = int64_t(blockIdx.x) * C::kWarps + warp;
@@ -497,7 +509,7 @@ paged_decode_kernel(const DecodeParams p) {
       const int seg = min(blocks_left, cur.nblk - cur.blk);
       const bool ends_item = cur.blk + seg == cur.nblk;
       __syncwarp();  // the previous item's readers of the staging area are done
-      stage_new_token<T, QH>(
+      stage_new_token<T, QH, kD * C::kEltB>(
           qrow + int64_t(cur.kvh) * p.kv_mul * kD, hg, p.kv_mul,
           static_cast<const T*>(p.k_new) + (int64_t(cur.b) * p.num_kv_heads + cur.kvh) * kD,
           static_cast<const uint8_t*>(p.v_new) + (int64_t(cur.b) * p.num_kv_heads + cur.kvh) * (kD * C::kEltB),
@@ -1044,6 +1056,7 @@ inline int64_t counter_bytes(int num_q_heads, int num_kv_heads) {
   const int64_t items = int64_t(kMaxBatch) * num_kv_heads * ((kv_mul + qh - 1) / qh);
   return (items * 4 + 255) / 256 * 256;
 }
+// Query heads a warp of paged_decode_kernel serves, and the unit the workspace is laid out in.
 inline int heads_per_warp(int kv_mul) {
   if (kv_mul == 1) return 1;
   if (kv_mul == 2) return 2;
@@ -1054,6 +1067,9 @@ constexpr int kMaxSms = 160;  // upper bound used to size the workspace
 constexpr int kMaxWarpsPerCta = 16;
 constexpr int kMinPartialSlots = 2 * kMaxSms * kMaxWarpsPerCta;  // two per warp of the largest grid
 constexpr int kStatusBytes = 256;
+// Floats of a workspace slot of `heads` heads; the counters of the two-level assembly live in the
+// last slot of an area of kMinPartialSlots slots of heads_per_warp(kv_mul) heads.
+constexpr int slot_floats_of(int heads) { return heads * kD + 8; }
 
 // Tuning knob: 0 = default shape; set through kpx_internal_set_decode_variant.
 extern int g_decode_variant;
@@ -1116,33 +1132,13 @@ int launch_shape(const DecodeParams& p, cudaStream_t stream, int flags) {
   // Launches that the caller overlaps on the GPU (KPX_DECODE_OVERLAPPED) run as three small CTAs
   // per SM instead of one large one: an SM then takes up the next launch's work a third at a
   // time while the previous launch's last warps finish.  Alone, the large CTA is faster.
-  const bool overlapped = (flags & KPX_DECODE_OVERLAPPED) != 0;
-  if (sizeof(T) == 4) {
-    if (small_launch(p, QH, 6)) return launch_decode<T, QH, 6, 2, 8, true>(p, stream);
-    return overlapped ? launch_decode<T, QH, 2, 2, 8, false, 3>(p, stream)
-                      : launch_decode<T, QH, 6, 2, 8>(p, stream);
-  }
-  // tuning knob for experiments: 1 forces the three-small-CTAs form, 2 the one-large-CTA form
-  const bool small_ctas = (g_decode_variant & 3) == 1 ? true : ((g_decode_variant & 3) == 2 ? false : overlapped);
-  if (small_launch(p, QH, 12)) return launch_decode<T, QH, 12, 2, 16, true>(p, stream);
-  return small_ctas ? launch_decode<T, QH, 4, 2, 16, false, 3>(p, stream)
-                    : launch_decode<T, QH, 12, 2, 16>(p, stream);
+  if (small_launch(p, QH, 6)) return launch_decode<T, QH, 6, 2, 8, true>(p, stream);
+  return (flags & KPX_DECODE_OVERLAPPED) ? launch_decode<T, QH, 2, 2, 8, false, 3>(p, stream)
+                                         : launch_decode<T, QH, 6, 2, 8>(p, stream);
 }
 
-#ifdef KPX_DECODE_INSTANTIATE
-template <typename T>
-int dispatch_decode(const DecodeParams& p, cudaStream_t stream, int flags) {
-  switch (heads_per_warp(p.kv_mul)) {
-    case 1: return launch_shape<T, 1>(p, stream, flags);
-    case 2: return launch_shape<T, 2>(p, stream, flags);
-    default: return launch_shape<T, 4>(p, stream, flags);
-  }
-}
-
-#else
 template <typename T>
 int dispatch_decode(const DecodeParams& p, cudaStream_t stream, int flags);
-#endif
 
 }  // namespace decode
 }  // namespace kpx

@@ -22,14 +22,12 @@
 // work area, and prefill_merge_kernel combines the parts.
 // Every mbarrier wait is bounded; a role that gives up raises a CTA-wide flag that ends the
 // other roles' waits, TMEM is freed on every path and the workspace status word is raised.
-#include <cuda.h>  // CUtensorMap and the enums of cuTensorMapEncodeTiled (types only; no libcuda link)
-
 #include <algorithm>
 #include <atomic>
 #include <type_traits>
 #include <vector>
 
-#include "kpx_common.cuh"
+#include "kpx_tma.cuh"
 
 namespace kpx {
 namespace {
@@ -237,23 +235,6 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
   *abort_flag = 1;
   return false;
 }
-// Tiled TMA loads, each into this CTA's own shared memory: a box of the tensor map lands there,
-// 128-byte swizzled, and its bytes are counted on the mbarrier.
-__device__ __forceinline__ void tma_load_3d(void* dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
-      ::"r"(smem_u32(dst)), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_4d(void* dst, const void* tmap, int c0, int c1, int c2, int c3,
-                                            uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
-      "[%6];"
-      ::"r"(smem_u32(dst)), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
-      : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t addr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -822,37 +803,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-}  // namespace
-
-namespace {
-// cuTensorMapEncodeTiled, looked up through the runtime so that the library carries no link
-// dependency on the driver library.
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = [] {
-    void* f = nullptr;
-    cudaDriverEntryPointQueryResult res;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &res) != cudaSuccess ||
-        res != cudaDriverEntryPointSuccess)
-      f = nullptr;
-    return reinterpret_cast<EncodeTiledFn>(f);
-  }();
-  return fn;
-}
-// rank-n map of 16-bit elements, 128-byte swizzle; dims/box innermost first, strides in bytes
-// for dimensions 1..n-1
-bool make_map(CUtensorMap* map, int32_t dtype, const void* base, int rank, const cuuint64_t* dims,
-              const cuuint64_t* strides_b, const cuuint32_t* box) {
-  EncodeTiledFn fn = encode_tiled_fn();
-  if (!fn) return false;
-  const cuuint32_t ones[4] = {1, 1, 1, 1};
-  return fn(map, dtype == KPX_F16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
-            cuuint32_t(rank), const_cast<void*>(base), dims, strides_b, box, ones, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
 }  // namespace
 
 // -1: cut underfilled calls (default); 0: never; 2..4: always, into that many parts (tests).
