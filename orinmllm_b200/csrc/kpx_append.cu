@@ -262,36 +262,51 @@ __global__ void sin_cos_kernel(float* __restrict__ sin_cache, float* __restrict_
   }
 }
 
-// Copy-on-write: whole blocks, every layer, K and V.  One CTA-row of threads per
-// 16-byte vector; a block's (head) tiles are copied tile by tile so both the
-// paged and the strided layout work.
-__global__ void cow_copy_kernel(uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
-                                int32_t num_layers, int64_t layer_stride_bytes,
-                                const int32_t* __restrict__ src_ids,
-                                const int32_t* __restrict__ dst_ids, int32_t n, LayoutDev L) {
-  const int vec_per_row = L.head_size * L.elt_bytes / 16;
-  const int64_t vec_per_block = int64_t(vec_per_row) * L.block_size * L.num_kv_heads;
-  const int64_t total = vec_per_block * n * num_layers * 2;
-  for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total;
-       i += int64_t(gridDim.x) * blockDim.x) {
-    int64_t r = i;
-    int vi = int(r % vec_per_row);
-    r /= vec_per_row;
-    int tok = int(r % L.block_size);
-    r /= L.block_size;
-    int h = int(r % L.num_kv_heads);
-    r /= L.num_kv_heads;
-    int which = int(r & 1);
-    r >>= 1;
-    int layer = int(r % num_layers);
-    int pair = int(r / num_layers);
-    int64_t s = src_ids[pair], d = dst_ids[pair];
-    if (s < 0 || d < 0 || s == d) continue;
-    uint8_t* pool = (which ? v_pool : k_pool) + layer * layer_stride_bytes;
-    int64_t in_block = (int64_t(h) * L.head_stride + int64_t(tok) * L.token_stride) * L.elt_bytes + vi * 16;
-    const uint4* src = reinterpret_cast<const uint4*>(pool + s * L.block_stride * L.elt_bytes + in_block);
-    uint4* dst = reinterpret_cast<uint4*>(pool + d * L.block_stride * L.elt_bytes + in_block);
-    *dst = *src;
+// Copy-on-write: whole blocks, every layer, K and V.  One CTA copies kCowVecs 16-byte vectors per
+// thread of one (pair, layer, K or V) block, all loads before the first store, so that what a CTA
+// does once (which block, which pool, the two ids) is off the path of the data; a block that is
+// one run of memory (the paged pool's) needs no index arithmetic per vector at all.  255 blocks of
+// 36 layers (1.2 GB moved): 268 -> 179 us, 6.7 TB/s; before, one flat index per vector took seven
+// 64-bit divisions apart.
+constexpr int kCowThreads = 256, kCowVecs = 4;
+__global__ void __launch_bounds__(kCowThreads)
+cow_copy_kernel(uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool, int32_t num_layers,
+                int64_t layer_stride_bytes, const int32_t* __restrict__ src_ids,
+                const int32_t* __restrict__ dst_ids, int64_t work, int64_t parts, int64_t vec_per_block, LayoutDev L) {
+  const uint32_t vec_per_row = uint32_t(L.head_size * L.elt_bytes / 16);
+  const bool one_run = L.token_stride == L.head_size &&
+                       (L.num_kv_heads == 1 || L.head_stride == int64_t(L.block_size) * L.head_size);
+  for (int64_t c = blockIdx.x; c < work; c += gridDim.x) {
+    // c = ((pair * layers + layer) * 2 + K or V) * parts + part
+    const int64_t block = c / parts;
+    const int64_t part = c - block * parts;
+    const int64_t pl = block >> 1;
+    const int64_t pair = pl / num_layers;
+    const int layer = int(pl - pair * num_layers);
+    const int64_t from = src_ids[pair], to = dst_ids[pair];
+    if (from < 0 || to < 0 || from == to) continue;
+    uint8_t* pool = ((block & 1) ? v_pool : k_pool) + layer * layer_stride_bytes;
+    const uint8_t* src = pool + from * L.block_stride * L.elt_bytes;
+    uint8_t* dst = pool + to * L.block_stride * L.elt_bytes;
+    uint4 val[kCowVecs];
+    int64_t off[kCowVecs];
+#pragma unroll
+    for (int u = 0; u < kCowVecs; ++u) {
+      const int64_t v = (part * kCowVecs + u) * kCowThreads + threadIdx.x;
+      off[u] = -1;
+      if (v >= vec_per_block) continue;
+      if (one_run) {
+        off[u] = v * 16;
+      } else {
+        const int64_t row = (vec_per_block >> 31) ? v / vec_per_row : int64_t(uint32_t(v) / vec_per_row);
+        const int64_t h = (vec_per_block >> 31) ? row / L.block_size : int64_t(uint32_t(row) / uint32_t(L.block_size));
+        off[u] = (h * L.head_stride + (row - h * L.block_size) * L.token_stride) * L.elt_bytes + (v - row * vec_per_row) * 16;
+      }
+      val[u] = *reinterpret_cast<const uint4*>(src + off[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < kCowVecs; ++u)
+      if (off[u] >= 0) *reinterpret_cast<uint4*>(dst + off[u]) = val[u];
   }
 }
 
@@ -486,11 +501,13 @@ extern "C" int kpx_cow_copy_blocks(void* k_pool, void* v_pool, const kpx_kv_layo
   if (!device_info().ok) return KPX_ERR_CUDA;
   LayoutDev L = to_dev(layout);
   if ((layer_stride * L.elt_bytes) % 16) return KPX_ERR_INVALID_ARGUMENT;
-  int64_t work = int64_t(L.head_size * L.elt_bytes / 16) * L.block_size * L.num_kv_heads * n * num_layers * 2;
-  const int threads = 256;
-  cow_copy_kernel<<<grid_for(work, threads), threads, 0, static_cast<cudaStream_t>(stream)>>>(
+  const int64_t vecs = int64_t(L.head_size * L.elt_bytes / 16) * L.block_size * L.num_kv_heads;
+  const int64_t parts = (vecs + kCowThreads * kCowVecs - 1) / (kCowThreads * kCowVecs);
+  const int64_t work = parts * n * num_layers * 2;
+  const int64_t grid = work < (int64_t(1) << 30) ? work : (int64_t(1) << 30);
+  cow_copy_kernel<<<unsigned(grid), kCowThreads, 0, static_cast<cudaStream_t>(stream)>>>(
       static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool), num_layers,
-      layer_stride * L.elt_bytes, src_ids, dst_ids, n, L);
+      layer_stride * L.elt_bytes, src_ids, dst_ids, work, parts, vecs, L);
   return cuda_status(cudaGetLastError());
 }
 
