@@ -113,6 +113,15 @@ __global__ void rope_append_kernel(T* __restrict__ q, T* __restrict__ k, const T
                                    const int64_t* __restrict__ slot_mapping, int32_t num_tokens,
                                    LayoutDev L, const float* __restrict__ q_norm_w,
                                    const float* __restrict__ k_norm_w, float norm_eps) {
+  const int64_t after_wait = grid_wait();
+  grid_release();
+  q += q ? after_wait : 0;
+  k += k ? after_wait : 0;
+  v += v ? after_wait : 0;
+  positions += positions ? after_wait : 0;
+  slot_mapping += slot_mapping ? after_wait : 0;
+  sin_cache += after_wait;
+  cos_cache += after_wait;
   constexpr int E = Elt<T>::kPer16B;
   const int hs = L.head_size;
   const int groups_per_head = hs / 2 / E;  // pair-groups per head
@@ -218,6 +227,12 @@ append_token_kernel(uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
                     const uint8_t* __restrict__ k_src, const uint8_t* __restrict__ v_src,
                     const int64_t* __restrict__ slot_mapping, const int32_t* __restrict__ pos_dev,
                     int32_t pos_bias, int32_t num_tokens, LayoutDev L) {
+  const int64_t after_wait = grid_wait();
+  grid_release();
+  k_src += after_wait;
+  v_src += v_src ? after_wait : 0;
+  slot_mapping += slot_mapping ? after_wait : 0;
+  pos_dev += pos_dev ? after_wait : 0;
   const int vec_per_head = L.head_size * L.elt_bytes / 16;
   const int vec_per_tok = vec_per_head * L.num_kv_heads;
   const int r = threadIdx.x;
@@ -400,12 +415,10 @@ extern "C" int kpx_append(void* k_pool, void* v_pool, const kpx_kv_layout* layou
   const int per_tok = int(work / num_tokens);
   if (per_tok <= 1024) {
     const int threads = (per_tok + 31) / 32 * 32;
-    append_token_kernel<<<token_grid(append_token_kernel, num_tokens, threads), threads, 0,
-                          static_cast<cudaStream_t>(stream)>>>(
-        static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool),
-        static_cast<const uint8_t*>(k_src), static_cast<const uint8_t*>(v_src), slot_mapping, pos_dev,
-        pos_bias, num_tokens, L);
-    return cuda_status(cudaGetLastError());
+    return launch_chained(append_token_kernel, dim3(token_grid(append_token_kernel, num_tokens, threads)), dim3(threads), 0,
+                          static_cast<cudaStream_t>(stream), static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool),
+                          static_cast<const uint8_t*>(k_src), static_cast<const uint8_t*>(v_src), slot_mapping, pos_dev,
+                          pos_bias, num_tokens, L);
   }
   const int threads = 256;
   append_kernel<<<grid_for((work + kAppendUnroll - 1) / kAppendUnroll, threads), threads, 0,
@@ -431,11 +444,10 @@ static int launch_rope(void* q, void* k, const void* v, int32_t q_heads, const i
                   ((v && v_pool) ? L.num_kv_heads * L.head_size / E : 0));
   if (work == 0) return KPX_OK;
   const int threads = 256;
-  rope_append_kernel<T><<<resident_grid_for(rope_append_kernel<T>, work, threads), threads, 0, stream>>>(
-      static_cast<T*>(q), static_cast<T*>(k), static_cast<const T*>(v), q_heads, positions, pos_base,
-      sin_cache, cos_cache, static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool),
-      slot_mapping, num_tokens, L, q_norm_w, k_norm_w, norm_eps);
-  return cuda_status(cudaGetLastError());
+  return launch_chained(rope_append_kernel<T>, dim3(resident_grid_for(rope_append_kernel<T>, work, threads)), dim3(threads), 0,
+                        stream, static_cast<T*>(q), static_cast<T*>(k), static_cast<const T*>(v), q_heads, positions, pos_base,
+                        sin_cache, cos_cache, static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool), slot_mapping,
+                        num_tokens, L, q_norm_w, k_norm_w, norm_eps);
 }
 
 extern "C" int kpx_rope_append(void* q, void* k, const void* v, int32_t q_heads,

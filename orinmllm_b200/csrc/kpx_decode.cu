@@ -87,6 +87,8 @@ __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeP
   __shared__ int prefix[kMaxBatch + 1];
   __shared__ int bad;
   const int tid = threadIdx.x;
+  grid_wait();
+  grid_release();
   if (tid == 0) bad = 0;
   for (int b = tid; b < p.batch; b += kPlanThreads) {
     prefix[b + 1] = blocks_of(seq_len_of(p, b));
@@ -183,9 +185,8 @@ extern "C" int kpx_decode_plan(void* plan, int64_t plan_bytes, const kpx_kv_layo
   int sms = device_info().sm_count;
   if (sms > kMaxSms) sms = kMaxSms;
   const int workers = sms * (layout->dtype == KPX_F32 ? 6 : kMmaWarpsPerSm);
-  decode_plan_kernel<<<(workers + kPlanThreads - 1) / kPlanThreads, kPlanThreads, 0, s>>>(
-      p, static_cast<int32_t*>(plan), workers);
-  return cuda_status(cudaGetLastError());
+  return launch_chained(decode_plan_kernel, dim3((workers + kPlanThreads - 1) / kPlanThreads), dim3(kPlanThreads), 0, s, p,
+                        static_cast<int32_t*>(plan), workers);
 }
 
 extern "C" int kpx_paged_decode_planned(void* out, const void* q, const void* k_pool, const void* v_pool,

@@ -344,6 +344,8 @@ paged_decode_kernel(const DecodeParams p) {
     for (int s = 0; s < 2 * NS; ++s) mbar_init(bars + s, 1);
     mbar_fence_init();
   }
+  const int64_t after_wait = grid_wait();
+  if (CPS == 1) grid_release();  // (launches that overlap others leave the SMs to those)
   // With a plan of the step the prefix and this warp's starting point come from it: one round
   // trip to global memory instead of lengths -> prefix -> search -> first block id.
   bool planned = false;
@@ -353,10 +355,11 @@ paged_decode_kernel(const DecodeParams p) {
       // header, this warp's entry and the prefix are requested together (a plan buffer always
       // holds kMaxSms x 16 entries and kMaxBatch + 1 prefix words, whatever was planned); what
       // the header says decides afterwards whether they are used
-      const int4 h = __ldg(reinterpret_cast<const int4*>(p.plan));
-      const int32_t plan_error = __ldg(p.plan + 4);
-      plan_entry = __ldg(reinterpret_cast<const int4*>(p.plan + kPlanEntriesAt) + (blockIdx.x * C::kWarps + warp));
-      for (int b = tid; b <= p.batch; b += C::kThreads) prefix[b] = __ldg(p.plan + kPlanPrefixAt + b);
+      const int32_t* plan = p.plan + after_wait;
+      const int4 h = __ldg(reinterpret_cast<const int4*>(plan));
+      const int32_t plan_error = __ldg(plan + 4);
+      plan_entry = __ldg(reinterpret_cast<const int4*>(plan + kPlanEntriesAt) + (blockIdx.x * C::kWarps + warp));
+      for (int b = tid; b <= p.batch; b += C::kThreads) prefix[b] = __ldg(plan + kPlanPrefixAt + b);
       planned = h.x == kPlanMark && h.y == p.batch && h.z == int(gridDim.x) * C::kWarps &&
                 h.w == p.num_kv_heads * p.head_groups;
       if (planned && blockIdx.x == 0 && tid == 0 && plan_error != 0) atomicMax(p.status, plan_error);
@@ -1116,9 +1119,7 @@ int launch_decode_form(DecodeParams p, cudaStream_t stream) {
   if (grid > kMaxSms) grid = kMaxSms;
   grid *= CPS;
   p.head_groups = (p.kv_mul + QH - 1) / QH;
-  kern<<<grid, C::kThreads, smem_bytes, stream>>>(p);
-  KPX_CUDA_TRY(cudaGetLastError());
-  return cuda_status(cudaGetLastError());
+  return launch_chained(kern, dim3(grid), dim3(C::kThreads), smem_bytes, stream, p);
 }
 
 template <typename T, int QH, int NW, int NS, int LPT, bool kSmall = false, int CPS = 1>

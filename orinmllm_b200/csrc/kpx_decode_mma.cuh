@@ -127,6 +127,8 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
     prefetch_tensormap(&map_k);
     prefetch_tensormap(&map_v);
   }
+  const int64_t after_wait = grid_wait();
+  if (CPS == 1) grid_release();  // (launches that overlap others leave the SMs to those)
   // With a plan of the step the prefix and this warp's starting point come from it: one round
   // trip to global memory instead of lengths -> prefix -> search -> first block id.
   bool planned = false;
@@ -136,10 +138,11 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
       // header, this warp's entry and the prefix are requested together (a plan buffer always
       // holds kMaxSms x 16 entries and kMaxBatch + 1 prefix words, whatever was planned); what
       // the header says decides afterwards whether they are used
-      const int4 h = __ldg(reinterpret_cast<const int4*>(p.plan));
-      const int32_t plan_error = __ldg(p.plan + 4);
-      plan_entry = __ldg(reinterpret_cast<const int4*>(p.plan + kPlanEntriesAt) + (blockIdx.x * NW + warp));
-      for (int b = tid; b <= p.batch; b += C::kThreads) prefix[b] = __ldg(p.plan + kPlanPrefixAt + b);
+      const int32_t* plan = p.plan + after_wait;
+      const int4 h = __ldg(reinterpret_cast<const int4*>(plan));
+      const int32_t plan_error = __ldg(plan + 4);
+      plan_entry = __ldg(reinterpret_cast<const int4*>(plan + kPlanEntriesAt) + (blockIdx.x * NW + warp));
+      for (int b = tid; b <= p.batch; b += C::kThreads) prefix[b] = __ldg(plan + kPlanPrefixAt + b);
       planned = h.x == kPlanMark && h.y == p.batch && h.z == int(gridDim.x) * NW &&
                 h.w == p.num_kv_heads * p.head_groups;
       if (planned && blockIdx.x == 0 && tid == 0 && plan_error != 0) atomicMax(p.status, plan_error);
@@ -673,8 +676,7 @@ int launch_mma_form(const DecodeParams& p, cudaStream_t stream) {
   if (!make_pool_map(&map_k, dtype, p.k_pool, p) || !make_pool_map(&map_v, dtype, p.v_pool, p)) return KPX_ERR_CUDA;
   int grid = device_info().sm_count;
   if (grid > kMaxSms) grid = kMaxSms;
-  kern<<<grid * CPS, C::kThreads, smem_bytes, stream>>>(p, map_k, map_v);
-  return cuda_status(cudaGetLastError());
+  return launch_chained(kern, dim3(grid * CPS), dim3(C::kThreads), smem_bytes, stream, p, map_k, map_v);
 }
 
 // Launches that the caller overlaps on the GPU (KPX_DECODE_OVERLAPPED) run as two CTAs of four

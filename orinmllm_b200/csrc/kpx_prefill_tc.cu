@@ -478,6 +478,8 @@ template <typename T>
 __global__ void __launch_bounds__(kD* kMergeRowLanes)
     prefill_merge_kernel(T* __restrict__ out, const float* __restrict__ partials, const MergeDesc* __restrict__ descs,
                          int num_q_heads) {
+  descs += grid_wait();
+  grid_release();
   const MergeDesc md = descs[blockIdx.x];
   const int d = threadIdx.x;
 #pragma unroll
@@ -540,6 +542,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   float* s_half = reinterpret_cast<float*>(sV + 2 * kOperandB + 256);  // [2 items][2][128]
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  grid_wait();
+  grid_release();
   const PairDesc pd = p.pairs[blockIdx.x];
   const int last_pos = pd.it[1].pos0 + pd.it[1].nrows - 1;  // newest position any row of the pair may see
   const int kv_len = last_pos + 1;
@@ -968,19 +972,17 @@ int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool,
       KPX_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes));
       if (dev < 64) done_mask->fetch_or(bit, std::memory_order_release);
     }
-    kernel<<<grid, kThreads, kSmemBytes, stream>>>(p, map_q, map_k, map_v);
-    return cuda_status(cudaGetLastError());
+    return launch_chained(kernel, dim3(grid), dim3(kThreads), kSmemBytes, stream, p, map_q, map_k, map_v);
   };
   static std::atomic<uint64_t> done_f16{0}, done_bf16{0};
   const int rc = layout->dtype == KPX_F16 ? launch(prefill_tc_kernel<__half>, &done_f16)
                                           : launch(prefill_tc_kernel<__nv_bfloat16>, &done_bf16);
   if (rc != KPX_OK || merges.empty()) return rc;
   const MergeDesc* md = reinterpret_cast<const MergeDesc*>(area + pair_bytes);
-  if (layout->dtype == KPX_F16)
-    prefill_merge_kernel<__half><<<dim3(unsigned(merges.size()), kTile / kMergeRowsPerCta), dim3(kD, kMergeRowLanes), 0, stream>>>(static_cast<__half*>(out), p.partials, md, num_q_heads);
-  else
-    prefill_merge_kernel<__nv_bfloat16><<<dim3(unsigned(merges.size()), kTile / kMergeRowsPerCta), dim3(kD, kMergeRowLanes), 0, stream>>>(static_cast<__nv_bfloat16*>(out), p.partials, md, num_q_heads);
-  return cuda_status(cudaGetLastError());
+  const dim3 mgrid(unsigned(merges.size()), kTile / kMergeRowsPerCta), mblock(kD, kMergeRowLanes);
+  return layout->dtype == KPX_F16
+             ? launch_chained(prefill_merge_kernel<__half>, mgrid, mblock, 0, stream, static_cast<__half*>(out), p.partials, md, num_q_heads)
+             : launch_chained(prefill_merge_kernel<__nv_bfloat16>, mgrid, mblock, 0, stream, static_cast<__nv_bfloat16*>(out), p.partials, md, num_q_heads);
 }
 
 // Bytes of the work area prefill_tc may need for a call with total_q query tokens.
