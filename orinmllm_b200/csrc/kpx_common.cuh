@@ -84,19 +84,28 @@ __device__ __forceinline__ int64_t grid_wait() {
 }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... P, typename... A>
-inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream,
-                          A&&... args) {
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+inline int launch_chained_cluster(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem_bytes, unsigned cluster,
+                                  cudaStream_t stream, A&&... args) {
+  cudaLaunchAttribute attr[2] = {};
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem_bytes;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
   return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+}
+template <typename... P, typename... A>
+inline int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem_bytes, cudaStream_t stream,
+                          A&&... args) {
+  return launch_chained_cluster(kernel, grid, block, smem_bytes, 1, stream, static_cast<A&&>(args)...);
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {

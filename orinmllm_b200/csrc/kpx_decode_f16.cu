@@ -1,5 +1,5 @@
 // Decode kernels for __half pools: the one place dispatch_decode<__half> is defined.
-#include "kpx_decode_mma.cuh"
+#include "kpx_decode_cluster.cuh"
 
 namespace kpx {
 namespace decode {

@@ -98,6 +98,7 @@ struct DecodeParams {
 // the sequence, id of that block); sequence 0xffff = the warp has no blocks.
 constexpr int32_t kPlanMark = 0x4b50504c;
 constexpr int kPlanPrefixAt = 8, kPlanEntriesAt = kPlanPrefixAt + kMaxBatch + 8, kPlanEntryWords = 4;
+constexpr int kMaxSms = 160;  // upper bound used to size the workspace
 
 template <typename T, int QH, int NW, int NS, int LPT>
 struct Cfg {
@@ -1066,7 +1067,6 @@ inline int heads_per_warp(int kv_mul) {
   return 4;
 }
 
-constexpr int kMaxSms = 160;  // upper bound used to size the workspace
 constexpr int kMaxWarpsPerCta = 16;
 constexpr int kMinPartialSlots = 2 * kMaxSms * kMaxWarpsPerCta;  // two per warp of the largest grid
 constexpr int kStatusBytes = 256;
@@ -1080,19 +1080,23 @@ extern int g_decode_variant;
 // is below g_small_below blocks per warp of the grid; then ranges hold at least
 // g_min_blocks_per_range blocks while at least g_min_warps_per_sm warps per SM stay active.
 extern int g_small_below, g_min_blocks_per_range, g_min_warps_per_sm;
+// Most blocks a warp takes in the cluster form of a small launch (0: form off).
+extern int g_cluster_share;
 extern uint32_t g_wait_limit;
 extern int g_withhold_worker;
 
-// True when the launch certainly has fewer than g_small_below blocks per warp.  What bounds a
-// sequence's blocks on the host: the table width; without a table (the reference's contiguous
-// cache) the fixed length if there is one, else the cache's size if the layout states it.
+// Most blocks a sequence of the launch can have, as far as the host can tell: the table width;
+// without a table (the reference's contiguous cache) the fixed length if there is one, else the
+// cache's size if the layout states it; -1 = unknown.
+inline int64_t seq_blocks_bound(const DecodeParams& p) {
+  if (p.block_table) return p.max_blocks_per_seq;
+  if (!p.seq_lens) return (int64_t(p.len_bias) + kBS - 1) / kBS;
+  return p.num_blocks > 0 ? p.num_blocks : -1;
+}
+// True when the launch certainly has fewer than g_small_below blocks per warp.
 inline bool small_launch(const DecodeParams& p, int qh, int warps_per_cta) {
-  if (g_small_below <= 0) return false;
-  int64_t per_seq_blocks;
-  if (p.block_table) per_seq_blocks = p.max_blocks_per_seq;
-  else if (!p.seq_lens) per_seq_blocks = (int64_t(p.len_bias) + kBS - 1) / kBS;
-  else if (p.num_blocks > 0) per_seq_blocks = p.num_blocks;
-  else return false;
+  const int64_t per_seq_blocks = seq_blocks_bound(p);
+  if (g_small_below <= 0 || per_seq_blocks < 0) return false;
   int grid = device_info().sm_count;
   if (grid > kMaxSms) grid = kMaxSms;
   const int64_t groups = (p.kv_mul + qh - 1) / qh;
@@ -1126,16 +1130,6 @@ template <typename T, int QH, int NW, int NS, int LPT, bool kSmall = false, int 
 int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   return p.k_new ? launch_decode_form<T, QH, NW, NS, LPT, kSmall, CPS, true>(p, stream)
                  : launch_decode_form<T, QH, NW, NS, LPT, kSmall, CPS, false>(p, stream);
-}
-
-template <typename T, int QH>
-int launch_shape(const DecodeParams& p, cudaStream_t stream, int flags) {
-  // Launches that the caller overlaps on the GPU (KPX_DECODE_OVERLAPPED) run as three small CTAs
-  // per SM instead of one large one: an SM then takes up the next launch's work a third at a
-  // time while the previous launch's last warps finish.  Alone, the large CTA is faster.
-  if (small_launch(p, QH, 6)) return launch_decode<T, QH, 6, 2, 8, true>(p, stream);
-  return (flags & KPX_DECODE_OVERLAPPED) ? launch_decode<T, QH, 2, 2, 8, false, 3>(p, stream)
-                                         : launch_decode<T, QH, 6, 2, 8>(p, stream);
 }
 
 template <typename T>

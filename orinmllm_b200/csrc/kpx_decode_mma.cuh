@@ -20,11 +20,6 @@
 // elements], one 4 KB box), so that ldmatrix reads them without bank conflicts.  A strided cache
 // may end inside a block: the rows of such a block that exist come by one bulk copy each, unswizzled.
 // Eight warps per SM with three K and three V slots each (192 KB of shared memory in flight).
-//
-// Measured, one layer of 64 sequences of 128..4096 tokens: 28/4 heads bf16 106 -> 64 us (262 MB;
-// 4.1 TB/s), 32/8 heads fp16 unchanged at 103..110 us (554 MB; 5.2 TB/s, bound by HBM and the
-// launch's ends); 256 sequences that share 1024 of 1344 tokens, 32/8: 228 -> 165 us.  Errors against
-// 64 bits are those of the output's rounding, as before (fp16 2.1e-4, bf16 1.7e-3).
 #pragma once
 #include "kpx_decode_impl.cuh"
 #include "kpx_tma.cuh"
@@ -81,6 +76,191 @@ struct Mma<__nv_bfloat16> {
   }
   static __device__ __forceinline__ float2 unpack(uint32_t w) {
     return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+  }
+};
+
+// One warp's part of one item: query rows, running softmax state and accumulator of eight heads, and
+// the arithmetic of a 16-token tile.
+template <typename T_>
+struct MmaTile {
+  using T = T_;
+  using M = Mma<T>;
+  static constexpr int QH = kMmaHeads, kRowB = kD * 2;
+  // rows of a staging area in shared memory: the stride spreads the eight rows that a warp reads
+  // at a time over the banks
+  static constexpr int kRowStride = kRowB + 16;
+  static constexpr bool kTensorMaps = true;
+  uint32_t qa[8][2];  // A fragments: k step s holds d = 16s + 2t, +1 and 16s + 8 + 2t, +1 of head g
+  float acc[16][4];   // d = 8 * tile + 2t, +1 of head g: [0..1] the P_hi part, [2..3] the P_lo part
+  float m, l;         // of head g; l: of the thread's own tokens until finish()
+  uint32_t hi[2], lo[2];  // weights of the block whose output pass comes next
+  int g, t;               // head; position in the quad
+  // ldmatrix addresses: lane 8m + r names row r of matrix m.  K: matrix m = 16-byte chunk m (mod 4)
+  // of tokens r; V: matrix m = tokens (m & 1) * 8 + r, chunk m >> 1 (mod 2).
+  int lm, lr;
+  uint32_t k_off, v_off;
+
+  __device__ __forceinline__ void reset() {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
+    m = -INFINITY;
+    l = 0.f;
+  }
+  __device__ __forceinline__ void init(int lane) {
+    g = lane >> 2;
+    t = lane & 3;
+    lm = lane >> 3;
+    lr = lane & 7;
+    k_off = uint32_t(lr * 128 + ((lm ^ lr) << 4));
+    v_off = uint32_t(((lm & 1) * 8 + lr) * 128 + (((lm >> 1) ^ lr) << 4));
+    reset();
+  }
+  // rows of the group's heads, `stride` bytes apart; heads from `heads` on are zero
+  __device__ __forceinline__ void load_q(const uint8_t* rows, int stride, int heads, float) {
+    const bool valid = g < heads;
+    const uint32_t* qh = reinterpret_cast<const uint32_t*>(rows + (valid ? g : 0) * stride) + t;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      qa[s][0] = valid ? qh[8 * s] : 0u;
+      qa[s][1] = valid ? qh[8 * s + 4] : 0u;
+    }
+  }
+  __device__ __forceinline__ int token(int e) const { return 2 * t + (e & 1) + (e >> 1) * 8; }
+  // Scores and weights of the block whose K tile is at kt; kTail: only nvalid of its tokens exist
+  // (linear: its rows lie one after the other, not swizzled).
+  template <bool kTail>
+  __device__ __forceinline__ void scores_of(uint32_t kt, int nvalid, bool linear, float qscale) {
+    float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};  // tokens 0..7, 8..15
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t a = kt + (k_off ^ ((i & 1) << 6)) + (i >> 1) * 2048, step8 = 1024;
+      if (kTail && linear) {
+        a = kt + lr * kRowB + (4 * i + lm) * 16;
+        step8 = 8 * kRowB;
+      }
+      uint32_t b0[4], b1[4];
+      ldsm4(b0, a);
+      ldsm4(b1, a + step8);
+      M::run(c0, qa[2 * i][0], 0u, qa[2 * i][1], 0u, b0[0], b0[1]);
+      M::run(c1, qa[2 * i][0], 0u, qa[2 * i][1], 0u, b1[0], b1[1]);
+      M::run(c0, qa[2 * i + 1][0], 0u, qa[2 * i + 1][1], 0u, b0[2], b0[3]);
+      M::run(c1, qa[2 * i + 1][0], 0u, qa[2 * i + 1][1], 0u, b1[2], b1[3]);
+    }
+    float s[4] = {c0[0] * qscale, c0[1] * qscale, c1[0] * qscale, c1[1] * qscale};
+    if (kTail) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (token(e) >= nvalid) s[e] = -INFINITY;
+    }
+    float mx = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    const float m_new = fmaxf(m, mx);
+    const float alpha = fast_exp2(m - m_new);
+    const bool changed = m_new != m;
+    m = m_new;
+    float w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      w[e] = fast_exp2(s[e] - m_new + M::kWeightBias);
+      if (kTail && token(e) >= nvalid) w[e] = 0.f;
+    }
+    l = l * alpha + ((w[0] + w[1]) + (w[2] + w[3]));
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      hi[h] = M::pack(w[2 * h], w[2 * h + 1]);
+      const float2 f = M::unpack(hi[h]);
+      lo[h] = M::pack(w[2 * h] - f.x, w[2 * h + 1] - f.y);
+    }
+    if (__any_sync(0xffffffffu, changed)) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] *= alpha;
+    }
+  }
+  // Output pass of that block, V tile at vt.
+  template <bool kTail>
+  __device__ __forceinline__ void output_of(uint32_t vt, int nvalid, bool linear) {
+    // rows past the newest token hold anything, NaN included: their halves of the packed pairs are cleared
+    uint32_t mask[2] = {0xffffffffu, 0xffffffffu};
+    if (kTail) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        mask[h] = (token(2 * h) < nvalid ? 0xffffu : 0u) | (token(2 * h + 1) < nvalid ? 0xffff0000u : 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint32_t a = vt + (v_off ^ ((i & 3) << 5)) + (i >> 2) * 2048;
+      if (kTail && linear) a = vt + ((lm & 1) * 8 + lr) * kRowB + (2 * i + (lm >> 1)) * 16;
+      uint32_t b[4];
+      ldsm4_trans(b, a);
+      if (kTail) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) b[e] &= mask[e & 1];
+      }
+      M::run(acc[2 * i], hi[0], lo[0], hi[1], lo[1], b[0], b[1]);
+      M::run(acc[2 * i + 1], hi[0], lo[0], hi[1], lo[1], b[2], b[3]);
+    }
+  }
+  __device__ __forceinline__ void scores(const uint8_t* kt, int nvalid, bool linear, float qscale) {
+    if (nvalid < kBS) scores_of<true>(smem_u32(kt), nvalid, linear, qscale);
+    else scores_of<false>(smem_u32(kt), nvalid, false, qscale);
+  }
+  __device__ __forceinline__ void output(const uint8_t* vt, int nvalid, bool linear) {
+    if (nvalid < kBS) output_of<true>(smem_u32(vt), nvalid, linear);
+    else output_of<false>(smem_u32(vt), nvalid, false);
+  }
+  // l over the head's tokens, in all four threads of the quad; acc[i][0..1] = the sum of both parts
+  __device__ __forceinline__ void finish() {
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      acc[i][0] += acc[i][2];
+      acc[i][1] += acc[i][3];
+    }
+  }
+  // after finish(): one more token whose rows are at k_row and v_row
+  __device__ __forceinline__ void add_token(const uint8_t* k_row, const uint8_t* v_row, float qscale) {
+    const uint32_t* kr = reinterpret_cast<const uint32_t*>(k_row) + t;
+    const uint32_t* vr = reinterpret_cast<const uint32_t*>(v_row) + t;
+    float s = 0.f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float2 a = M::unpack(qa[i][h]), b = M::unpack(kr[8 * i + 4 * h]);
+        s = fmaf(a.x, b.x, fmaf(a.y, b.y, s));
+      }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    s *= qscale;
+    const float m_new = fmaxf(m, s);
+    const float a = fast_exp2(m - m_new), w = fast_exp2(s - m_new + M::kWeightBias);
+    m = m_new;
+    l = l * a + w;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float2 v = M::unpack(vr[4 * i]);
+      acc[i][0] = fmaf(w, v.x, acc[i][0] * a);
+      acc[i][1] = fmaf(w, v.y, acc[i][1] * a);
+    }
+  }
+  // after finish(): [heads][128] accumulators, then the maxima, then the sums
+  __device__ __forceinline__ void store(float* dst, int heads = kMmaHeads) const {
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      *reinterpret_cast<float2*>(dst + g * kD + 8 * i + 2 * t) = make_float2(acc[i][0], acc[i][1]);
+    if (t == 0) {
+      dst[heads * kD + g] = m;
+      dst[heads * kD + heads + g] = l;
+    }
+  }
+  static __device__ __forceinline__ void write4(T* row, int d, float4 v) {
+    *reinterpret_cast<uint2*>(row + d) = make_uint2(M::pack(v.x, v.y), M::pack(v.z, v.w));
   }
 };
 
@@ -179,12 +359,9 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
   if (u0 >= u1) return;  // nothing below synchronises across warps
   const int n = int(u1 - u0);
 
-  const int g = lane >> 2, t = lane & 3;  // head of the group; position in the quad
-  // ldmatrix addresses: lane 8m + r names row r of matrix m.  K: matrix m = 16-byte chunk m (mod 4)
-  // of tokens r; V: matrix m = tokens (m & 1) * 8 + r, chunk m >> 1 (mod 2).
-  const int lm = lane >> 3, lr = lane & 7;
-  const uint32_t k_off = uint32_t(lr * 128 + ((lm ^ lr) << 4));
-  const uint32_t v_off = uint32_t(((lm & 1) * 8 + lr) * 128 + (((lm >> 1) ^ lr) << 4));
+  MmaTile<T> tile;
+  tile.init(lane);
+  const int g = tile.g, t = tile.t;  // head of the group; position in the quad
 
   // ---- producer side: block ids and tile requests of this warp's own range; one cursor walks
   // the range NS blocks ahead of the consumer ----
@@ -199,18 +376,10 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
   } else {
     cur.locate(p, prefix, u0);
   }
-  // Query rows of the current item as A fragments: k step s holds d = 16s + 2t, +1 and 16s + 8 + 2t, +1.
-  uint32_t qa[8][2];
   auto load_q = [&]() {
-    const int hq = (cur.sub - cur.kvh * p.head_groups) * kMmaHeads + g;
-    const bool valid = hq < p.kv_mul;
-    const uint32_t* qh = reinterpret_cast<const uint32_t*>(
-        static_cast<const T*>(p.q) + (int64_t(cur.b) * p.num_q_heads + cur.kvh * p.kv_mul + (valid ? hq : 0)) * kD) + t;
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      qa[s][0] = valid ? __ldg(qh + 8 * s) : 0u;
-      qa[s][1] = valid ? __ldg(qh + 8 * s + 4) : 0u;
-    }
+    const int h0 = (cur.sub - cur.kvh * p.head_groups) * kMmaHeads;
+    tile.load_q(static_cast<const uint8_t*>(p.q) + (int64_t(cur.b) * p.num_q_heads + cur.kvh * p.kv_mul + h0) * kRowB, kRowB,
+                p.kv_mul - h0, p.qscale);
   };
   // The first item's rows are requested here, before the first block id and the first tiles, so
   // that their latency (DRAM if nothing brought them to L2) runs under those.
@@ -268,8 +437,6 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
   }
 
   // ---- consumer state ----
-  float acc[16][4];  // d = 8 * tile + 2t, +1 of head g: [0..1] the P_hi part, [2..3] the P_lo part
-  float m_run, l_run;
   auto begin_item = [&](int blocks_left, bool first) {
     if constexpr (kFused) {
       const int hg = cur.sub - cur.kvh * p.head_groups;
@@ -283,22 +450,11 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
           p.sin_cache + int64_t(cur.len) * kD, p.cos_cache + int64_t(cur.len) * kD,
           cur.row ? cur.row + cur.len / kBS : nullptr, cur.len / kBS, stage, lane);
       __syncwarp();
-      const bool valid = hg * kMmaHeads + g < p.kv_mul;
-      const uint32_t* qh = reinterpret_cast<const uint32_t*>(stage + g * C::kRowStride) + t;
-#pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        qa[s][0] = valid ? qh[8 * s] : 0u;
-        qa[s][1] = valid ? qh[8 * s + 4] : 0u;
-      }
+      tile.load_q(stage, C::kRowStride, p.kv_mul - hg * kMmaHeads, p.qscale);
     } else if (!first) {
       load_q();
     }
-#pragma unroll
-    for (int i = 0; i < 16; ++i)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[i][e] = 0.f;
-    m_run = -INFINITY;
-    l_run = 0.f;
+    tile.reset();
   };
 
   auto end_item = [&](const Cursor& item, bool whole_item, int64_t partial_slot, int64_t item_start,
@@ -306,41 +462,11 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
     const int hg = item.sub - item.kvh * p.head_groups;
     const int hq = hg * kMmaHeads + g;  // this thread's head within the KV head
     const bool head_ok = hq < p.kv_mul;
-    float l = l_run;  // of head g, in all four threads of the quad
-    l += __shfl_xor_sync(0xffffffffu, l, 1);
-    l += __shfl_xor_sync(0xffffffffu, l, 2);
-    float m = m_run;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      acc[i][0] += acc[i][2];
-      acc[i][1] += acc[i][3];
-    }
+    tile.finish();
     if (kFused && has_item_end) {
       // Fused step: this piece ends the item, so it also carries the new token (position
       // item.len, not in the pool yet), staged when the item began.
-      const uint32_t* kr = reinterpret_cast<const uint32_t*>(stage + kMmaHeads * C::kRowStride) + t;
-      const uint32_t* vr = reinterpret_cast<const uint32_t*>(stage + (kMmaHeads + 1) * C::kRowStride) + t;
-      float s = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const float2 a = M::unpack(qa[i][h]), b = M::unpack(kr[8 * i + 4 * h]);
-          s = fmaf(a.x, b.x, fmaf(a.y, b.y, s));
-        }
-      s += __shfl_xor_sync(0xffffffffu, s, 1);
-      s += __shfl_xor_sync(0xffffffffu, s, 2);
-      s *= p.qscale;
-      const float m_new = fmaxf(m, s);
-      const float a = fast_exp2(m - m_new), w = fast_exp2(s - m_new + M::kWeightBias);
-      m = m_new;
-      l = l * a + w;
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const float2 v = M::unpack(vr[4 * i]);
-        acc[i][0] = fmaf(w, v.x, acc[i][0] * a);
-        acc[i][1] = fmaf(w, v.y, acc[i][1] * a);
-      }
+      tile.add_token(stage + kMmaHeads * C::kRowStride, stage + (kMmaHeads + 1) * C::kRowStride, p.qscale);
       // append: the first head group's warp stores the rows (lanes 0..15 the K row, 16..31 the V
       // row) into the block that holds position item.len
       if (hg == 0) {
@@ -358,26 +484,17 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
     T* orow = static_cast<T*>(p.out) + (int64_t(item.b) * p.num_q_heads + item.kvh * p.kv_mul + hq) * kD;
     if (whole_item) {
       if (head_ok) {
-        const float inv = 1.f / l;
+        const float inv = 1.f / tile.l;
         uint32_t* o = reinterpret_cast<uint32_t*>(orow) + t;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) o[4 * i] = M::pack(acc[i][0] * inv, acc[i][1] * inv);
+        for (int i = 0; i < 16; ++i) o[4 * i] = M::pack(tile.acc[i][0] * inv, tile.acc[i][1] * inv);
       }
       return;
     }
     // one workspace slot: slot_heads accumulators of 128, then their maxima, then their sums
     const int sh = p.slot_heads;
     const int64_t slot_floats = sh > 4 ? 2 * slot_floats_of(4) : slot_floats_of(sh);
-    if (head_ok) {
-      float* ps = p.partials + partial_slot * slot_floats;
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-        *reinterpret_cast<float2*>(ps + g * kD + 8 * i + 2 * t) = make_float2(acc[i][0], acc[i][1]);
-      if (t == 0) {
-        ps[sh * kD + g] = m;
-        ps[sh * kD + sh + g] = l;
-      }
-    }
+    if (head_ok) tile.store(p.partials + partial_slot * slot_floats, sh);
     // The item is cut by a range boundary.  Publish this piece, then count it; the warp
     // that brings the count up to the number of pieces assembles the item from all of
     // them (nobody waits: whoever arrives last does the work) and resets the counter.
@@ -506,88 +623,14 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
     constexpr bool kTail = decltype(tail_tag)::value;
     const bool linear = kTail && !p.tile_contig;  // rows copied one by one, not swizzled
     if (!wait_slot(bars + slot, phase)) return false;
-    float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};  // tokens 0..7, 8..15
-    {
-      const uint32_t kt = ring_u + slot * C::kTileB;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        uint32_t a = kt + (k_off ^ ((i & 1) << 6)) + (i >> 1) * 2048, step8 = 1024;
-        if (linear) {
-          a = kt + lr * kRowB + (4 * i + lm) * 16;
-          step8 = 8 * kRowB;
-        }
-        uint32_t b0[4], b1[4];
-        ldsm4(b0, a);
-        ldsm4(b1, a + step8);
-        M::run(c0, qa[2 * i][0], 0u, qa[2 * i][1], 0u, b0[0], b0[1]);
-        M::run(c1, qa[2 * i][0], 0u, qa[2 * i][1], 0u, b1[0], b1[1]);
-        M::run(c0, qa[2 * i + 1][0], 0u, qa[2 * i + 1][1], 0u, b0[2], b0[3]);
-        M::run(c1, qa[2 * i + 1][0], 0u, qa[2 * i + 1][1], 0u, b1[2], b1[3]);
-      }
-    }
+    tile.template scores_of<kTail>(ring_u + slot * C::kTileB, nvalid, linear, p.qscale);
     __syncwarp();  // the K slot is read
     if (k_issued < n) {
       if (lane == 0) fence_proxy_async();
       issue_k(slot);
     }
-    float s[4] = {c0[0] * p.qscale, c0[1] * p.qscale, c1[0] * p.qscale, c1[1] * p.qscale};
-    const int tok[4] = {2 * t, 2 * t + 1, 2 * t + 8, 2 * t + 9};
-    if (kTail) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (tok[e] >= nvalid) s[e] = -INFINITY;
-    }
-    float mx = fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-    mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-    const float m_new = fmaxf(m_run, mx);
-    const float alpha = fast_exp2(m_run - m_new);
-    const bool changed = m_new != m_run;
-    m_run = m_new;
-    float w[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      w[e] = fast_exp2(s[e] - m_new + M::kWeightBias);
-      if (kTail && tok[e] >= nvalid) w[e] = 0.f;
-    }
-    l_run = l_run * alpha + ((w[0] + w[1]) + (w[2] + w[3]));
-    uint32_t hi[2], lo[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      hi[h] = M::pack(w[2 * h], w[2 * h + 1]);
-      const float2 f = M::unpack(hi[h]);
-      lo[h] = M::pack(w[2 * h] - f.x, w[2 * h + 1] - f.y);
-    }
-    if (__any_sync(0xffffffffu, changed)) {
-#pragma unroll
-      for (int i = 0; i < 16; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[i][e] *= alpha;
-    }
     if (!wait_slot(bars + NS + slot, phase)) return false;
-    {
-      const uint32_t vt = ring_u + (NS + slot) * C::kTileB;
-      // rows past the newest token hold anything, NaN included: their halves of the packed pairs are cleared
-      uint32_t mask[2] = {0xffffffffu, 0xffffffffu};
-      if (kTail) {
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-          mask[h] = (tok[2 * h] < nvalid ? 0xffffu : 0u) | (tok[2 * h + 1] < nvalid ? 0xffff0000u : 0u);
-      }
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        uint32_t a = vt + (v_off ^ ((i & 3) << 5)) + (i >> 2) * 2048;
-        if (linear) a = vt + ((lm & 1) * 8 + lr) * kRowB + (2 * i + (lm >> 1)) * 16;
-        uint32_t b[4];
-        ldsm4_trans(b, a);
-        if (kTail) {
-#pragma unroll
-          for (int e = 0; e < 4; ++e) b[e] &= mask[e & 1];
-        }
-        M::run(acc[2 * i], hi[0], lo[0], hi[1], lo[1], b[0], b[1]);
-        M::run(acc[2 * i + 1], hi[0], lo[0], hi[1], lo[1], b[2], b[3]);
-      }
-    }
+    tile.template output_of<kTail>(ring_u + (NS + slot) * C::kTileB, nvalid, linear);
     __syncwarp();  // the V slot is read
     if (v_issued < n) {
       if (lane == 0) fence_proxy_async();
@@ -677,22 +720,6 @@ int launch_mma_form(const DecodeParams& p, cudaStream_t stream) {
   int grid = device_info().sm_count;
   if (grid > kMaxSms) grid = kMaxSms;
   return launch_chained(kern, dim3(grid * CPS), dim3(C::kThreads), smem_bytes, stream, p, map_k, map_v);
-}
-
-// Launches that the caller overlaps on the GPU (KPX_DECODE_OVERLAPPED) run as two CTAs of four
-// warps per SM instead of one of eight: an SM then takes up the next launch's work a half at a
-// time while the previous launch's last warps finish.
-template <typename T>
-int dispatch_decode_mma(DecodeParams p, cudaStream_t stream, int flags) {
-  p.head_groups = (p.kv_mul + kMmaHeads - 1) / kMmaHeads;
-  p.small = small_launch(p, kMmaHeads, kMmaWarpsPerSm) ? 1 : 0;
-  p.slot_heads = p.kv_mul > 4 ? kMmaHeads : heads_per_warp(p.kv_mul);
-  // eight-head slots are twice a four-head slot
-  if (p.slot_heads == kMmaHeads) p.partial_slots /= 2;
-  const bool overlapped = (g_decode_variant & 3) == 1 ? true : ((g_decode_variant & 3) == 2 ? false : (flags & KPX_DECODE_OVERLAPPED) != 0);
-  const bool small_ctas = overlapped && !p.small;
-  if (p.k_new) return small_ctas ? launch_mma_form<T, 4, 3, 2, true>(p, stream) : launch_mma_form<T, 8, 3, 1, true>(p, stream);
-  return small_ctas ? launch_mma_form<T, 4, 3, 2, false>(p, stream) : launch_mma_form<T, 8, 3, 1, false>(p, stream);
 }
 
 }  // namespace decode
