@@ -7,6 +7,7 @@ Produces, next to this file under ``lib/``:
   libkpx.so          CUDA kernels + the C ABI declared in include/kpx.h
   libkuiper_b200.so  C++ host layer (kuiper-style op::Layer adapters, kernel registry,
                      block pool manager, radix tree / prefix cache) on top of libkpx
+  _kpx_py.so         CPython binding of the entry points that a step calls once per layer
 The CPU checker under ``oracle/`` and the C++ test program are test infrastructure and are
 built by tests/buildtools.py, not from here.
 """
@@ -17,6 +18,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG = Path(__file__).resolve().parent
@@ -114,6 +116,16 @@ def build_host(force=False, verbose=False) -> Path | None:
     return so
 
 
+def build_py(force=False, verbose=False) -> Path:
+    """csrc/python/kpx_py.c (CPython binding of the per-layer entry points) -> lib/_kpx_py.so."""
+    src = CSRC / "python" / "kpx_py.c"
+    so = LIB / "_kpx_py.so"
+    if force or _newer(so, [src] + _headers() + [LIB / "libkpx.so"]):
+        _run(["gcc", "-O2", "-std=c11", "-fPIC", "-shared", "-Wall", "-fvisibility=hidden", "-I", INCLUDE,
+              "-I", sysconfig.get_paths()["include"], "-o", so, src, f"-L{LIB}", "-lkpx", "-Wl,-rpath,$ORIGIN"], verbose)
+    return so
+
+
 def _nccl_dirs():
     """(include dir, library file) of the NCCL this process would load: the one packaged with the
     Python environment if there is one (torch loads that), else the system's."""
@@ -155,6 +167,7 @@ def build_comm(force=False, verbose=False) -> Path | None:
 def build_all(force=False, verbose=False, ptxas_info=False):
     build_kpx(force, verbose, ptxas_info)
     build_host(force, verbose)
+    build_py(force, verbose)
     build_comm(force, verbose)
 
 

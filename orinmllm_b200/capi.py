@@ -1,8 +1,9 @@
-"""ctypes binding of the C ABI in include/kpx.h (lib/libkpx.so).
+"""Binding of the C ABI in include/kpx.h (lib/libkpx.so).
 
 This is a thin loader for test drivers, the benchmark and Python callers: every
 function forwards raw device pointers to the native library and raises on a
-non-zero status.  There is no Python or CPU implementation behind it: if the
+non-zero status.  What a step calls once per layer goes through lib/_kpx_py.so
+(csrc/python/kpx_py.c), the rest through ctypes.  There is no Python or CPU implementation behind it: if the
 native library has not been built, importing `lib()` raises.
 """
 from __future__ import annotations
@@ -98,6 +99,41 @@ def lib() -> C.CDLL:
     return _lib
 
 
+_py = None
+
+
+def _entries():
+    """Load lib/_kpx_py.so (once).  Raises if it has not been built."""
+    global _py
+    if _py is None:
+        import importlib.machinery
+        import importlib.util
+        lib()
+        path = LIB_DIR / "_kpx_py.so"
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: build the native libraries first "
+                               "(python -m orinmllm_b200.build); there is no fallback path")
+        loader = importlib.machinery.ExtensionFileLoader("_kpx_py", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_kpx_py", loader))
+        loader.exec_module(module)
+        module.set_stream_source(_current_device, _raw_stream)
+        _py = module
+    return _py
+
+
+def _current_device() -> int:
+    """The first call makes torch set CUDA up; the next ones ask its C functions directly."""
+    import torch
+    device = torch.cuda.current_device()
+    _py.set_stream_source(torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream)
+    return device
+
+
+def _raw_stream(device: int) -> int:
+    import torch
+    return torch.cuda.current_stream(device).cuda_stream
+
+
 def status_string(status: int) -> str:
     return lib().kpx_status_string(int(status)).decode()
 
@@ -154,24 +190,21 @@ def append(k_pool, v_pool, layout, k_src, v_src, slot_mapping=None, pos_dev=None
            num_tokens=None, stream=None) -> None:
     if num_tokens is None:
         num_tokens = k_src.shape[0]
-    check(lib().kpx_append(ptr(k_pool), ptr(v_pool), C.byref(layout), ptr(k_src), ptr(v_src),
-                           ptr(slot_mapping), ptr(pos_dev), pos_bias, num_tokens, _stream(stream)),
-          "kpx_append")
+    check((_py or _entries()).append(k_pool, v_pool, layout, k_src, v_src, slot_mapping, pos_dev, pos_bias,
+                                     num_tokens, stream), "kpx_append")
 
 
 def rope_append(q, k, v, q_heads, positions, sin_cache, cos_cache, k_pool, v_pool, layout,
                 slot_mapping, num_tokens, stream=None, pos_base=0) -> None:
-    check(lib().kpx_rope_append(ptr(q), ptr(k), ptr(v), q_heads, ptr(positions), pos_base, ptr(sin_cache),
-                                ptr(cos_cache), ptr(k_pool), ptr(v_pool), C.byref(layout),
-                                ptr(slot_mapping), num_tokens, _stream(stream)), "kpx_rope_append")
+    check((_py or _entries()).rope_append(q, k, v, q_heads, positions, pos_base, sin_cache, cos_cache, k_pool,
+                                          v_pool, layout, slot_mapping, num_tokens, stream), "kpx_rope_append")
 
 
 def norm_rope_append(q, k, v, q_heads, q_norm_weight, k_norm_weight, norm_eps, positions, sin_cache, cos_cache,
                      k_pool, v_pool, layout, slot_mapping, num_tokens, stream=None, pos_base=0) -> None:
-    check(lib().kpx_norm_rope_append(ptr(q), ptr(k), ptr(v), q_heads, ptr(q_norm_weight), ptr(k_norm_weight),
-                                     norm_eps, ptr(positions), pos_base, ptr(sin_cache), ptr(cos_cache),
-                                     ptr(k_pool), ptr(v_pool), C.byref(layout), ptr(slot_mapping), num_tokens,
-                                     _stream(stream)), "kpx_norm_rope_append")
+    check((_py or _entries()).norm_rope_append(q, k, v, q_heads, q_norm_weight, k_norm_weight, norm_eps, positions,
+                                               pos_base, sin_cache, cos_cache, k_pool, v_pool, layout, slot_mapping,
+                                               num_tokens, stream), "kpx_norm_rope_append")
 
 
 def sin_cos_cache(sin_cache, cos_cache, head_size, max_seq_len, theta, stream=None) -> None:
@@ -197,10 +230,9 @@ def workspace_status(workspace, stream=None) -> int:
 def paged_decode(out, q, k_pool, v_pool, layout, block_table, max_blocks_per_seq, seq_lens,
                  len_bias, batch, num_q_heads, scale, workspace, workspace_bytes,
                  stream=None) -> None:
-    check(lib().kpx_paged_decode(ptr(out), ptr(q), ptr(k_pool), ptr(v_pool), C.byref(layout),
-                                 ptr(block_table), max_blocks_per_seq, ptr(seq_lens), len_bias,
-                                 batch, num_q_heads, scale, ptr(workspace), workspace_bytes,
-                                 _stream(stream)), "kpx_paged_decode")
+    check((_py or _entries()).paged_decode(out, q, k_pool, v_pool, layout, block_table, max_blocks_per_seq,
+                                           seq_lens, len_bias, batch, num_q_heads, scale, workspace,
+                                           workspace_bytes, stream), "kpx_paged_decode")
 
 
 KPX_DECODE_OVERLAPPED = 1
@@ -210,21 +242,20 @@ def rope_append_decode(out, q, k_new, v_new, sin_cache, cos_cache, k_pool, v_poo
                        max_blocks_per_seq, positions, batch, num_q_heads, scale, workspace,
                        workspace_bytes, flags=0, stream=None) -> None:
     """One decode step of a layer in one launch (RoPE + append + attention)."""
-    check(lib().kpx_rope_append_decode(ptr(out), ptr(q), ptr(k_new), ptr(v_new), ptr(sin_cache),
-                                       ptr(cos_cache), ptr(k_pool), ptr(v_pool), C.byref(layout),
-                                       ptr(block_table), max_blocks_per_seq, ptr(positions), batch,
-                                       num_q_heads, scale, ptr(workspace), workspace_bytes, flags,
-                                       _stream(stream)), "kpx_rope_append_decode")
+    check((_py or _entries()).rope_append_decode(out, q, k_new, v_new, sin_cache, cos_cache, k_pool, v_pool, layout,
+                                                 block_table, max_blocks_per_seq, positions, batch, num_q_heads,
+                                                 scale, workspace, workspace_bytes, flags, stream),
+          "kpx_rope_append_decode")
 
 
 def paged_decode_overlapped(out, q, k_pool, v_pool, layout, block_table, max_blocks_per_seq, seq_lens,
                             len_bias, batch, num_q_heads, scale, workspace, workspace_bytes,
                             stream=None) -> None:
     """kpx_paged_decode in the form for launches that overlap on the GPU (own workspace each)."""
-    check(lib().kpx_paged_decode_overlapped(ptr(out), ptr(q), ptr(k_pool), ptr(v_pool), C.byref(layout),
-                                            ptr(block_table), max_blocks_per_seq, ptr(seq_lens), len_bias,
-                                            batch, num_q_heads, scale, ptr(workspace), workspace_bytes,
-                                            _stream(stream)), "kpx_paged_decode_overlapped")
+    check((_py or _entries()).paged_decode_overlapped(out, q, k_pool, v_pool, layout, block_table,
+                                                      max_blocks_per_seq, seq_lens, len_bias, batch, num_q_heads,
+                                                      scale, workspace, workspace_bytes, stream),
+          "kpx_paged_decode_overlapped")
 
 
 def decode_plan_bytes() -> int:
@@ -234,18 +265,17 @@ def decode_plan_bytes() -> int:
 def decode_plan(plan, plan_bytes, layout, block_table, max_blocks_per_seq, seq_lens, len_bias, batch,
                 num_q_heads, stream=None) -> None:
     """Works out once what every decode launch of a step would work out in its prologue."""
-    check(lib().kpx_decode_plan(ptr(plan), plan_bytes, C.byref(layout), ptr(block_table), max_blocks_per_seq,
-                                ptr(seq_lens), len_bias, batch, num_q_heads, _stream(stream)), "kpx_decode_plan")
+    check((_py or _entries()).decode_plan(plan, plan_bytes, layout, block_table, max_blocks_per_seq, seq_lens,
+                                          len_bias, batch, num_q_heads, stream), "kpx_decode_plan")
 
 
 def paged_decode_planned(out, q, k_pool, v_pool, layout, block_table, max_blocks_per_seq, seq_lens,
                          len_bias, batch, num_q_heads, scale, workspace, workspace_bytes, plan, flags=0,
                          stream=None) -> None:
     """kpx_paged_decode / _overlapped (by flags) with the step's plan."""
-    check(lib().kpx_paged_decode_planned(ptr(out), ptr(q), ptr(k_pool), ptr(v_pool), C.byref(layout),
-                                         ptr(block_table), max_blocks_per_seq, ptr(seq_lens), len_bias,
-                                         batch, num_q_heads, scale, ptr(workspace), workspace_bytes,
-                                         ptr(plan), flags, _stream(stream)), "kpx_paged_decode_planned")
+    check((_py or _entries()).paged_decode_planned(out, q, k_pool, v_pool, layout, block_table, max_blocks_per_seq,
+                                                   seq_lens, len_bias, batch, num_q_heads, scale, workspace,
+                                                   workspace_bytes, plan, flags, stream), "kpx_paged_decode_planned")
 
 
 def paged_decode_static(out, q, k_pool, v_pool, layout, block_table, max_blocks_per_seq, seq_lens,
@@ -267,10 +297,9 @@ def prefill_workspace_bytes(total_q, num_q_heads, num_kv_heads, head_size=128) -
 def paged_prefill(out, q, k_pool, v_pool, layout, block_table, max_blocks_per_seq, cu_q_lens_host,
                   start_pos_host, batch, num_q_heads, scale, workspace, workspace_bytes,
                   stream=None) -> None:
-    check(lib().kpx_paged_prefill(ptr(out), ptr(q), ptr(k_pool), ptr(v_pool), C.byref(layout),
-                                  ptr(block_table), max_blocks_per_seq, ptr(cu_q_lens_host),
-                                  ptr(start_pos_host), batch, num_q_heads, scale, ptr(workspace),
-                                  workspace_bytes, _stream(stream)), "kpx_paged_prefill")
+    check((_py or _entries()).paged_prefill(out, q, k_pool, v_pool, layout, block_table, max_blocks_per_seq,
+                                            cu_q_lens_host, start_pos_host, batch, num_q_heads, scale, workspace,
+                                            workspace_bytes, stream), "kpx_paged_prefill")
 
 
 def cow_copy_blocks(k_pool, v_pool, layout, num_layers, layer_stride, src_ids, dst_ids, n,

@@ -1,0 +1,72 @@
+"""The CPython binding (lib/_kpx_py.so) converts what the ctypes signatures convert and refuses what
+they refuse; no GPU is needed: the entry points check their arguments before they touch a device."""
+
+import numpy as np
+import pytest
+
+from orinmllm_b200 import capi
+
+
+@pytest.fixture()
+def entries(native_libs):
+    module = capi._entries()
+    module.set_stream_source(lambda: 0, lambda device: 0)
+    yield module
+    module.set_stream_source(capi._current_device, capi._raw_stream)
+
+
+def _decode(**change):
+    t = np.zeros(64, np.float32)
+    args = dict(out=t, q=t, k_pool=t, v_pool=t, layout=capi.layout_paged(capi.KPX_F32, 2), block_table=t,
+                max_blocks_per_seq=1, seq_lens=t, len_bias=0, batch=0, num_q_heads=2, scale=1.0, workspace=1 << 20,
+                workspace_bytes=1 << 40)
+    args.update(change)
+    capi.paged_decode(**args)
+
+
+class _Tensor:
+    def __init__(self, address):
+        self.address = address
+
+    def data_ptr(self):
+        return self.address
+
+
+def test_accepted(entries):
+    _decode()  # a batch of 0 is done without a device
+    _decode(out=4096, q=_Tensor(8192), scale=2, stream=np.int64(0))
+    _decode(batch=1 << 32)  # integers are cut to their width, as ctypes cuts them
+    _decode(workspace=_Tensor(256), block_table=None)
+
+
+@pytest.mark.parametrize("change", [dict(max_blocks_per_seq=1.0), dict(q="text"), dict(q=b"bytes"), dict(layout=None),
+                                    dict(layout=b"short"), dict(scale="1"), dict(batch=None), dict(q=_Tensor("x")),
+                                    dict(batch=np.int64(0))])
+def test_refused_before_the_call(entries, change):
+    with pytest.raises(TypeError):
+        _decode(**change)
+
+
+def test_status_becomes_an_error(entries):
+    with pytest.raises(capi.KpxError) as e:
+        _decode(out=None)
+    assert e.value.status == capi.KPX_ERR_INVALID_ARGUMENT
+    with pytest.raises(capi.KpxError) as e:
+        _decode(q=8)  # not 16-byte aligned: the address arrived as it is
+    assert e.value.status == capi.KPX_ERR_INVALID_ARGUMENT
+    with pytest.raises(capi.KpxError) as e:
+        _decode(workspace_bytes=16)
+    assert e.value.status == capi.KPX_ERR_WORKSPACE_TOO_SMALL
+
+
+def test_views_of_arrays_keep_their_address(entries):
+    t = np.zeros(64, np.float32)
+    first = 1 if t.ctypes.data % 16 == 0 else (16 - t.ctypes.data % 16) // 4 + 1
+    with pytest.raises(capi.KpxError):
+        _decode(q=t[first:])      # off a 16-byte boundary
+    _decode(q=t[first - 1::4])    # on one, strided
+
+
+def test_number_of_arguments(entries):
+    with pytest.raises(TypeError):
+        entries.paged_decode(1, 2, 3)
