@@ -710,7 +710,7 @@ def run_gpu(args):
                 "d2h_bytes_per_step": wl.d2h_bytes_per_step(), "ms_per_step": round(ms_e2e / K, 4),
                 "tokens_per_s": round(world * BATCH / (ms_e2e / K / 1e3), 1)},
         "gpu_launches": launches,
-        "roofline": {"bound": "hbm", "kernel": "paged_decode_kernel", "achieved": round(achieved, 1),
+        "roofline": {"bound": "hbm", "kernel": "paged_decode_mma_kernel", "achieved": round(achieved, 1),
                      "peak": peak, "peak_source": peak_src, "unit": "GB/s",
                      "frac": round(achieved / peak, 4), "avg_launch_us": round(in_region_ms * 1e3, 2),
                      "timed": "CUDA events around the timed region / decode launches inside it (launches of "
