@@ -19,7 +19,17 @@
 // Tiles arrive by TMA through 128-byte-swizzled tensor maps of the pools ([half row][16 tokens][64
 // elements], one 4 KB box), so that ldmatrix reads them without bank conflicts.  A strided cache
 // may end inside a block: the rows of such a block that exist come by one bulk copy each, unswizzled.
-// Eight warps per SM with three K and three V slots each (192 KB of shared memory in flight).
+// Eight warps per SM.  A launch that has the GPU to itself gives a warp one K and one V slot: 64 KB
+// in flight per SM keep HBM busy, and more only lengthens the queues, in which the SMs farther from
+// the memory they read fall behind until the last warp ends 25 us after the median one.  us per
+// launch with 1 / 2 / 3 slots: 32/8 heads, 64 sequences of 128..4096 tokens 100 / 104 / 110; 16 of
+// 8k..32k 215 / 226 / 237; one of 131072 107 / 110 / 113; 28/4 heads bf16, 64 sequences
+// 61 / 65 / 66.6.  (Twelve warps of two slots: 134; four warps of six: 126.)
+//
+// Measured, one layer of 64 sequences of 128..4096 tokens, before (packed FMAs) -> now: 28/4 heads
+// bf16 106 -> 61 us (277 MB; 4.5 TB/s), 32/8 heads fp16 105 -> 100 us (554 MB; 5.5 TB/s, bound by HBM
+// and the launch's ends); 256 sequences that share 1024 of 1344 tokens, 32/8: 228 -> 159 us.  Errors
+// against 64 bits are those of the output's rounding, as before (fp16 2.1e-4, bf16 1.7e-3).
 #pragma once
 #include "kpx_decode_impl.cuh"
 #include "kpx_tma.cuh"
