@@ -50,6 +50,8 @@ __device__ __forceinline__ void ldsm4_trans(uint32_t (&r)[4], uint32_t addr) {
                : "memory");
 }
 
+constexpr float kLeastHalf = 5.9604644775390625e-8f;  // 2^-24, the least positive fp16 value
+
 template <typename T>
 struct Mma;
 template <>
@@ -171,16 +173,18 @@ struct MmaTile {
     const float alpha = fast_exp2(m - m_new);
     const bool changed = m_new != m;
     m = m_new;
-    float w[4];
+    float w[4], first[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       w[e] = fast_exp2(s[e] - m_new + M::kWeightBias);
       if (kTail && token(e) >= nvalid) w[e] = 0.f;
+      // 0 only where the weight is (see finish()); a bf16 value reaches as low as a weight does
+      first[e] = std::is_same<T, __half>::value && w[e] > 0.f ? fmaxf(w[e], kLeastHalf) : w[e];
     }
     l = l * alpha + ((w[0] + w[1]) + (w[2] + w[3]));
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      hi[h] = M::pack(w[2 * h], w[2 * h + 1]);
+      hi[h] = M::pack(first[2 * h], first[2 * h + 1]);
       const float2 f = M::unpack(hi[h]);
       lo[h] = M::pack(w[2 * h] - f.x, w[2 * h + 1] - f.y);
     }
@@ -223,15 +227,19 @@ struct MmaTile {
     if (nvalid < kBS) output_of<true>(smem_u32(vt), nvalid, linear);
     else output_of<false>(smem_u32(vt), nvalid, false);
   }
-  // l over the head's tokens, in all four threads of the quad; acc[i][0..1] = the sum of both parts
+  // l over the head's tokens, in all four threads of the quad; acc[i][0..1] = the sum of both parts.
+  // Where V holds an infinity (fp16 caches overflow to one) the part of the first terms alone says
+  // what becomes of the sum, as no weight but 0 has a first term of 0.  A second term may be 0 or
+  // negative, so that its part is then an infinity of either sign or NaN; it is finite otherwise, and
+  // counts only if it is.
   __device__ __forceinline__ void finish() {
     l += __shfl_xor_sync(0xffffffffu, l, 1);
     l += __shfl_xor_sync(0xffffffffu, l, 2);
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      acc[i][0] += acc[i][2];
-      acc[i][1] += acc[i][3];
-    }
+    for (int i = 0; i < 16; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        if (fabsf(acc[i][2 + e]) < INFINITY) acc[i][e] += acc[i][2 + e];
   }
   // after finish(): one more token whose rows are at k_row and v_row
   __device__ __forceinline__ void add_token(const uint8_t* k_row, const uint8_t* v_row, float qscale) {
