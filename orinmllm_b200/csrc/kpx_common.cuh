@@ -11,12 +11,17 @@
 namespace kpx {
 
 // ---- host-side helpers ---------------------------------------------------------------
-inline int cuda_status(cudaError_t e) { return e == cudaSuccess ? KPX_OK : KPX_ERR_CUDA; }
+// The status of a runtime call.  An error is taken out of the runtime as well: left there, the next
+// launch that asks for the last error, this library's or the caller's, would report it as its own.
+inline int cuda_status(cudaError_t e) {
+  if (e == cudaSuccess) return KPX_OK;
+  (void)cudaGetLastError();
+  return KPX_ERR_CUDA;
+}
 
-#define KPX_CUDA_TRY(expr)                         \
-  do {                                             \
-    cudaError_t kpx_e__ = (expr);                  \
-    if (kpx_e__ != cudaSuccess) return KPX_ERR_CUDA; \
+#define KPX_CUDA_TRY(expr)                                                        \
+  do {                                                                            \
+    if (const int kpx_rc__ = ::kpx::cuda_status(expr)) return kpx_rc__;           \
   } while (0)
 
 inline int elt_bytes(int32_t dtype) { return dtype == KPX_F32 ? 4 : 2; }

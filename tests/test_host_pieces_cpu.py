@@ -1,0 +1,15 @@
+"""Small pieces of the launch path's host code, compiled by themselves and run without a GPU."""
+import subprocess
+from pathlib import Path
+
+from orinmllm_b200 import build as b
+
+CPP = Path(__file__).resolve().parent / "cpp"
+
+
+def test_a_refused_launch_leaves_no_error_behind(tmp_path):
+    exe = tmp_path / "launch_error"
+    subprocess.run([b._nvcc(), *b.NVCC_FLAGS, "-o", exe, CPP / "test_launch_error.cu", "-Xlinker",
+                    "--wrap=cudaLaunchKernelExC", "-Xlinker", "--wrap=cudaGetLastError"], check=True)
+    run = subprocess.run([exe], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout
