@@ -18,6 +18,7 @@
 // FmaTile (fp32 caches, packed FMAs).
 #pragma once
 #include "kpx_decode_mma.cuh"
+#include "kpx_once.h"
 
 namespace kpx {
 namespace decode {
@@ -444,25 +445,20 @@ template <typename Tile, int NW, int NS, bool kFused>
 const ClusterForm* cluster_form() {
   using C = ClusterCfg<Tile, NW, NS>;
   constexpr int smem_bytes = kFused ? C::kSmemFused : C::kSmem;
-  static ClusterForm forms[64];
-  static std::atomic<uint64_t> done{0};
-  static std::mutex mu;
+  static PerDevice<ClusterForm> forms;
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  const uint64_t bit = uint64_t(1) << dev;
-  if (!(done.load(std::memory_order_acquire) & bit)) {
-    std::lock_guard<std::mutex> lock(mu);
-    ClusterForm& f = forms[dev];
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  return forms.get(dev, [](ClusterForm& f) {
     auto kern = decode_cluster_kernel<Tile, NW, NS, kFused>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
       (void)cudaGetLastError();
-      return nullptr;
+      return false;
     }
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, 32 * NW, smem_bytes) != cudaSuccess) {
       (void)cudaGetLastError();
-      return nullptr;
+      return false;
     }
     f.fit[0] = per_sm * device_info().sm_count;
     for (int i = 1; i <= 4; ++i) {
@@ -481,9 +477,8 @@ const ClusterForm* cluster_form() {
         f.fit[i] = 0;
       }
     }
-    done.fetch_or(bit, std::memory_order_release);
-  }
-  return &forms[dev];
+    return true;
+  });
 }
 
 // CTAs per item of a small launch in this form, 0 if it is not for it: all clusters run side by

@@ -13,3 +13,10 @@ def test_a_refused_launch_leaves_no_error_behind(tmp_path):
                     "--wrap=cudaLaunchKernelExC", "-Xlinker", "--wrap=cudaGetLastError"], check=True)
     run = subprocess.run([exe], capture_output=True, text=True)
     assert run.returncode == 0, run.stdout
+
+
+def test_a_device_value_is_worked_out_once(tmp_path):
+    exe = tmp_path / "per_device"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-pthread", "-I", b.CSRC, "-o", exe, CPP / "test_per_device.cpp"], check=True)
+    run = subprocess.run([exe], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout
