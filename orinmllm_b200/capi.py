@@ -117,6 +117,7 @@ def _entries():
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_kpx_py", loader))
         loader.exec_module(module)
         module.set_stream_source(_current_device, _raw_stream)
+        module.set_layout_type(KvLayout)
         _py = module
     return _py
 

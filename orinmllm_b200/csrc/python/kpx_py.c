@@ -18,6 +18,7 @@
 
 static PyObject *s_data_ptr, *s_ctypes, *s_data;
 static PyObject *get_device, *get_stream; /* callables given to set_stream_source */
+static PyObject* layout_type;             /* the type of a layout, given to set_layout_type */
 
 typedef struct {
   PyObject* const* at; /* next argument */
@@ -98,12 +99,17 @@ static kpx_kv_layout arg_layout(Args* a) {
   kpx_kv_layout l = {0};
   Py_buffer view;
   if (a->bad) return l;
+  if (!layout_type || !PyObject_TypeCheck(o, (PyTypeObject*)layout_type)) { /* (not any bytes of its size) */
+    PyErr_Format(PyExc_TypeError, "a KvLayout is expected, not %s", Py_TYPE(o)->tp_name);
+    a->bad = 1;
+    return l;
+  }
   if (PyObject_GetBuffer(o, &view, PyBUF_SIMPLE) != 0) {
     a->bad = 1;
     return l;
   }
-  if (view.len == (Py_ssize_t)sizeof l) {
-    l = *(const kpx_kv_layout*)view.buf;
+  if (view.len >= (Py_ssize_t)sizeof l) {
+    memcpy(&l, view.buf, sizeof l);
   } else {
     PyErr_SetString(PyExc_TypeError, "a KvLayout is expected");
     a->bad = 1;
@@ -193,12 +199,23 @@ static PyObject* set_stream_source(PyObject* self, PyObject* args) {
   Py_RETURN_NONE;
 }
 
+static PyObject* set_layout_type(PyObject* self, PyObject* type) {
+  (void)self;
+  if (!PyType_Check(type)) {
+    PyErr_SetString(PyExc_TypeError, "a type is expected");
+    return NULL;
+  }
+  Py_XSETREF(layout_type, Py_NewRef(type));
+  Py_RETURN_NONE;
+}
+
 #define METHOD(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, NULL}
 static PyMethodDef methods[] = {METHOD(append), METHOD(rope_append), METHOD(norm_rope_append), METHOD(paged_decode),
                                 METHOD(paged_decode_overlapped), METHOD(paged_decode_planned), METHOD(decode_plan),
                                 METHOD(rope_append_decode), METHOD(paged_prefill),
                                 {"set_stream_source", set_stream_source, METH_VARARGS,
                                  "(current device, raw stream of a device): what a stream of None stands for"},
+                                {"set_layout_type", set_layout_type, METH_O, "the type that a layout argument is of"},
                                 {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_kpx_py", NULL, -1, methods, NULL, NULL, NULL, NULL};
 

@@ -1,6 +1,8 @@
 """The CPython binding (lib/_kpx_py.so) converts what the ctypes signatures convert and refuses what
 they refuse; no GPU is needed: the entry points check their arguments before they touch a device."""
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -45,6 +47,28 @@ def test_accepted(entries):
 def test_refused_before_the_call(entries, change):
     with pytest.raises(TypeError):
         _decode(**change)
+
+
+class _Other(ctypes.Structure):
+    _fields_ = capi.KvLayout._fields_
+
+
+class _Longer(capi.KvLayout):
+    _fields_ = [("note", ctypes.c_int64)]
+
+
+@pytest.mark.parametrize("layout", [bytes(bytearray(ctypes.sizeof(capi.KvLayout))), _Other(), (ctypes.c_int64 * 6)(),
+                                    np.zeros(6, np.int64)], ids=["bytes", "structure", "array", "numpy"])
+def test_only_a_layout_is_a_layout(entries, layout):
+    """Memory of the layout's size, with a layout's contents even, is not taken for one."""
+    assert memoryview(layout).nbytes == ctypes.sizeof(capi.KvLayout)
+    if isinstance(layout, ctypes.Structure):
+        ctypes.memmove(ctypes.byref(layout), ctypes.byref(capi.layout_paged(capi.KPX_F32, 2)), ctypes.sizeof(layout))
+    with pytest.raises(TypeError):
+        _decode(layout=layout)
+    longer = _Longer()
+    ctypes.memmove(ctypes.byref(longer), ctypes.byref(capi.layout_paged(capi.KPX_F32, 2)), ctypes.sizeof(capi.KvLayout))
+    _decode(layout=longer)  # a type derived from it is one
 
 
 def test_status_becomes_an_error(entries):
