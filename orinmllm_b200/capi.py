@@ -118,8 +118,22 @@ def _entries():
         loader.exec_module(module)
         module.set_stream_source(_current_device, _raw_stream)
         module.set_layout_type(KvLayout)
+        module.set_number_source(_number)
         _py = module
     return _py
+
+
+def _number(kind: int, value):
+    """What ctypes takes for a number besides numbers: a scalar of the argument's own type, or an object
+    whose _as_parameter_ is one."""
+    ctype = (_I32, _I64, _F32)[kind]
+    while hasattr(value, "_as_parameter_"):
+        value = value._as_parameter_
+    if isinstance(value, ctype):
+        return value.value
+    if isinstance(value, (int, float) if ctype is _F32 else int):
+        return value
+    raise TypeError(f"{ctype.__name__} or a number expected instead of {type(value).__name__}")
 
 
 def _current_device() -> int:

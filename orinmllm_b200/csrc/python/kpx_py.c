@@ -7,7 +7,7 @@
  * tensor, one data_ptr() call: about 1 us a call.  28 layers of a 512-token fp32 chat (56 calls)
  * took 587 us before and 279 us now, 28 fused steps of 8 short sequences 439 and 273 us.  Conversions accept what the ctypes signatures accept: None, int or
  * an object with data_ptr() / ctypes.data for a pointer, int for an integer (cut to its width), a
- * number for a float, a ctypes structure for the layout.  The GIL is released around the call.
+ * number for a float, a ctypes scalar of the argument's type for either, a KvLayout for the layout.  The GIL is released around the call.
  */
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
@@ -19,6 +19,8 @@
 static PyObject *s_data_ptr, *s_ctypes, *s_data;
 static PyObject *get_device, *get_stream; /* callables given to set_stream_source */
 static PyObject* layout_type;             /* the type of a layout, given to set_layout_type */
+static PyObject* get_number;              /* (kind, object) -> number, given to set_number_source */
+enum { KIND_I32, KIND_I64, KIND_F32 };
 
 typedef struct {
   PyObject* const* at; /* next argument */
@@ -71,26 +73,47 @@ static void* arg_ptr(Args* a) {
   Py_DECREF(v);
   return p;
 }
-static int64_t arg_i64(Args* a) {
+/* what is no plain number: a ctypes scalar or an object that stands for one, or a TypeError */
+static PyObject* number_of(PyObject* o, int kind, Args* a) {
+  PyObject* v = get_number ? PyObject_CallFunction(get_number, "iO", kind, o) : NULL;
+  if (!v) {
+    if (!PyErr_Occurred()) PyErr_Format(PyExc_TypeError, "a number is expected, not %s", Py_TYPE(o)->tp_name);
+    a->bad = 1;
+  }
+  return v;
+}
+static int64_t arg_int(Args* a, int kind) {
   PyObject* o = *a->at++;
   int64_t v;
   if (a->bad) return 0;
-  if (!PyLong_Check(o)) {
-    PyErr_Format(PyExc_TypeError, "int expected instead of %s", Py_TYPE(o)->tp_name);
-    a->bad = 1;
+  if (PyLong_Check(o)) {
+    Py_INCREF(o);
+  } else if (!(o = number_of(o, kind, a))) {
     return 0;
   }
   v = (int64_t)PyLong_AsUnsignedLongLongMask(o);
   if (PyErr_Occurred()) a->bad = 1;
+  Py_DECREF(o);
   return v;
 }
-static int32_t arg_i32(Args* a) { return (int32_t)arg_i64(a); }
+static int64_t arg_i64(Args* a) { return arg_int(a, KIND_I64); }
+static int32_t arg_i32(Args* a) { return (int32_t)arg_int(a, KIND_I32); }
 static float arg_f32(Args* a) {
   PyObject* o = *a->at++;
   double v;
   if (a->bad) return 0.f;
   v = PyFloat_AsDouble(o);
-  if (v == -1.0 && PyErr_Occurred()) a->bad = 1;
+  if (v == -1.0 && PyErr_Occurred()) {
+    if (!PyErr_ExceptionMatches(PyExc_TypeError)) {
+      a->bad = 1;
+      return 0.f;
+    }
+    PyErr_Clear();
+    if (!(o = number_of(o, KIND_F32, a))) return 0.f;
+    v = PyFloat_AsDouble(o);
+    if (PyErr_Occurred()) a->bad = 1;
+    Py_DECREF(o);
+  }
   return (float)v;
 }
 /* the layout is copied: nothing of the caller's is held while the GIL is released */
@@ -209,6 +232,12 @@ static PyObject* set_layout_type(PyObject* self, PyObject* type) {
   Py_RETURN_NONE;
 }
 
+static PyObject* set_number_source(PyObject* self, PyObject* source) {
+  (void)self;
+  Py_XSETREF(get_number, Py_NewRef(source));
+  Py_RETURN_NONE;
+}
+
 #define METHOD(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, NULL}
 static PyMethodDef methods[] = {METHOD(append), METHOD(rope_append), METHOD(norm_rope_append), METHOD(paged_decode),
                                 METHOD(paged_decode_overlapped), METHOD(paged_decode_planned), METHOD(decode_plan),
@@ -216,6 +245,8 @@ static PyMethodDef methods[] = {METHOD(append), METHOD(rope_append), METHOD(norm
                                 {"set_stream_source", set_stream_source, METH_VARARGS,
                                  "(current device, raw stream of a device): what a stream of None stands for"},
                                 {"set_layout_type", set_layout_type, METH_O, "the type that a layout argument is of"},
+                                {"set_number_source", set_number_source, METH_O,
+                                 "(0 int32, 1 int64, 2 float; object): the number that the object stands for"},
                                 {NULL, NULL, 0, NULL}};
 static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, "_kpx_py", NULL, -1, methods, NULL, NULL, NULL, NULL};
 

@@ -41,6 +41,24 @@ def test_accepted(entries):
     _decode(workspace=_Tensor(256), block_table=None)
 
 
+class _Holder:
+    def __init__(self, value):
+        self._as_parameter_ = value
+
+
+def test_ctypes_scalars(entries):
+    """A scalar of the argument's own ctypes type is the number it holds."""
+    _decode(batch=ctypes.c_int32(0), scale=ctypes.c_float(0.5), max_blocks_per_seq=_Holder(1), len_bias=_Holder(ctypes.c_int32(0)),
+            workspace_bytes=ctypes.c_int64(1 << 40))
+    with pytest.raises(capi.KpxError) as e:
+        _decode(workspace_bytes=ctypes.c_int64(16))
+    assert e.value.status == capi.KPX_ERR_WORKSPACE_TOO_SMALL
+    for change in (dict(batch=ctypes.c_int64(0)), dict(batch=ctypes.c_float(0)), dict(scale=ctypes.c_double(1)),
+                   dict(batch=_Holder("0")), dict(scale=_Holder("1"))):
+        with pytest.raises(TypeError):
+            _decode(**change)
+
+
 @pytest.mark.parametrize("change", [dict(max_blocks_per_seq=1.0), dict(q="text"), dict(q=b"bytes"), dict(layout=None),
                                     dict(layout=b"short"), dict(scale="1"), dict(batch=None), dict(q=_Tensor("x")),
                                     dict(batch=np.int64(0))])
