@@ -7,7 +7,7 @@ Produces, next to this file under ``lib/``:
   libkpx.so          CUDA kernels + the C ABI declared in include/kpx.h
   libkuiper_b200.so  C++ host layer (kuiper-style op::Layer adapters, kernel registry,
                      block pool manager, radix tree / prefix cache) on top of libkpx
-  _kpx_py.so         CPython binding of the entry points that a step calls once per layer
+  _kpx_py.<abi>.so   CPython binding of the entry points that a step calls once per layer
 The CPU checker under ``oracle/`` and the C++ test program are test infrastructure and are
 built by tests/buildtools.py, not from here.
 """
@@ -116,13 +116,23 @@ def build_host(force=False, verbose=False) -> Path | None:
     return so
 
 
-def build_py(force=False, verbose=False) -> Path:
-    """csrc/python/kpx_py.c (CPython binding of the per-layer entry points) -> lib/_kpx_py.so."""
+def py_binding() -> Path:
+    """Where the binding for the running interpreter lies: an extension is good for one version of
+    CPython only, and its name says which."""
+    return LIB / ("_kpx_py" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def build_py(force=False, verbose=False) -> Path | None:
+    """csrc/python/kpx_py.c (CPython binding of the per-layer entry points) -> lib/_kpx_py.<abi>.so.
+    Skipped (None) where this interpreter's headers are not installed: only Python callers need it."""
     src = CSRC / "python" / "kpx_py.c"
-    so = LIB / "_kpx_py.so"
+    include = Path(sysconfig.get_paths()["include"])
+    if not (include / "Python.h").exists():
+        return None
+    so = py_binding()
     if force or _newer(so, [src] + _headers() + [LIB / "libkpx.so"]):
         _run(["gcc", "-O2", "-std=c11", "-fPIC", "-shared", "-Wall", "-fvisibility=hidden", "-I", INCLUDE,
-              "-I", sysconfig.get_paths()["include"], "-o", so, src, f"-L{LIB}", "-lkpx", "-Wl,-rpath,$ORIGIN"], verbose)
+              "-I", include, "-o", so, src, f"-L{LIB}", "-lkpx", "-Wl,-rpath,$ORIGIN"], verbose)
     return so
 
 

@@ -2,8 +2,8 @@
 
 This is a thin loader for test drivers, the benchmark and Python callers: every
 function forwards raw device pointers to the native library and raises on a
-non-zero status.  What a step calls once per layer goes through lib/_kpx_py.so
-(csrc/python/kpx_py.c), the rest through ctypes.  There is no Python or CPU implementation behind it: if the
+non-zero status.  What a step calls once per layer goes through the extension module
+lib/_kpx_py.<abi>.so (csrc/python/kpx_py.c), the rest through ctypes.  There is no Python or CPU implementation behind it: if the
 native library has not been built, importing `lib()` raises.
 """
 from __future__ import annotations
@@ -103,15 +103,16 @@ _py = None
 
 
 def _entries():
-    """Load lib/_kpx_py.so (once).  Raises if it has not been built."""
+    """Load the extension built for this interpreter (once).  Raises if it has not been built."""
     global _py
     if _py is None:
         import importlib.machinery
         import importlib.util
+        import sysconfig
         lib()
-        path = LIB_DIR / "_kpx_py.so"
+        path = LIB_DIR / ("_kpx_py" + sysconfig.get_config_var("EXT_SUFFIX"))
         if not path.exists():
-            raise RuntimeError(f"{path} is missing: build the native libraries first "
+            raise RuntimeError(f"{path} is missing: build the native libraries first, with this interpreter and its headers "
                                "(python -m orinmllm_b200.build); there is no fallback path")
         loader = importlib.machinery.ExtensionFileLoader("_kpx_py", str(path))
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_kpx_py", loader))

@@ -1,4 +1,4 @@
-/* CPython binding of the entry points that a step calls once per layer (lib/_kpx_py.so).
+/* CPython binding of the entry points that a step calls once per layer (lib/_kpx_py.<abi>.so).
  *
  * A decode step of a short context is two launches of a few microseconds per layer, and calling
  * them through ctypes cost more than running them: about 4.5 us of argument conversion per call

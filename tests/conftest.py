@@ -35,7 +35,8 @@ def native_libs():
     """Build (if stale) and return the path of the CUDA library; building needs nvcc only."""
     from orinmllm_b200 import build
     so = build.LIB / "libkpx.so"
-    if not so.exists() or os.environ.get("KPX_REBUILD"):
+    # (a checkout built before, or with another interpreter, may have one and not the other)
+    if not so.exists() or not build.py_binding().exists() or os.environ.get("KPX_REBUILD"):
         build.build_all()
     if os.environ.get("KPX_DECODE_VARIANT"):
         import ctypes

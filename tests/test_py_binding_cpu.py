@@ -1,4 +1,4 @@
-"""The CPython binding (lib/_kpx_py.so) converts what the ctypes signatures convert and refuses what
+"""The CPython binding (lib/_kpx_py.<abi>.so) converts what the ctypes signatures convert and refuses what
 they refuse; no GPU is needed: the entry points check their arguments before they touch a device."""
 
 import ctypes
@@ -112,3 +112,21 @@ def test_views_of_arrays_keep_their_address(entries):
 def test_number_of_arguments(entries):
     with pytest.raises(TypeError):
         entries.paged_decode(1, 2, 3)
+
+
+def test_the_file_is_this_interpreters(native_libs, monkeypatch, tmp_path):
+    """The extension's name carries the interpreter's ABI, another interpreter's file is not loaded in
+    its place, and without Python.h everything else is built."""
+    import sysconfig
+    from orinmllm_b200 import build
+    assert build.py_binding().exists()
+    assert build.py_binding().name == "_kpx_py" + sysconfig.get_config_var("EXT_SUFFIX") != "_kpx_py.so"
+    monkeypatch.setattr(capi, "_py", None)
+    monkeypatch.setattr(capi, "LIB_DIR", tmp_path)
+    monkeypatch.setattr(capi, "lib", lambda: None)
+    for name in ("_kpx_py.so", "_kpx_py.cpython-399-x86_64-linux-gnu.so"):
+        (tmp_path / name).symlink_to(build.py_binding())
+    with pytest.raises(RuntimeError, match="build the native libraries"):
+        capi._entries()
+    monkeypatch.setattr(build.sysconfig, "get_paths", lambda: {"include": str(tmp_path)})
+    assert build.build_py(force=True) is None
