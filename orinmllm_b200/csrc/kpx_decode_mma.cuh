@@ -215,8 +215,20 @@ struct MmaTile {
 #pragma unroll
         for (int e = 0; e < 4; ++e) b[e] &= mask[e & 1];
       }
-      M::run(acc[2 * i], hi[0], lo[0], hi[1], lo[1], b[0], b[1]);
-      M::run(acc[2 * i + 1], hi[0], lo[0], hi[1], lo[1], b[2], b[3]);
+      // The products of a tile are summed by themselves and added to the running sums in fp32, rounded
+      // to nearest: a matrix instruction cuts its sums off, and over hundreds of tiles that adds up.
+      float d[2][4] = {};
+#pragma unroll
+      for (int u = 0; u < 2; ++u) M::run(d[u], hi[0], lo[0], hi[1], lo[1], b[2 * u], b[2 * u + 1]);
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int e = 0; e < 4; e += 2) {
+          float(&a)[4] = acc[2 * i + u];
+          const float2 sum = __fadd2_rn(make_float2(a[e], a[e + 1]), make_float2(d[u][e], d[u][e + 1]));
+          a[e] = sum.x;
+          a[e + 1] = sum.y;
+        }
     }
   }
   __device__ __forceinline__ void scores(const uint8_t* kt, int nvalid, bool linear, float qscale) {

@@ -1,6 +1,5 @@
-"""Decode attention of 16-bit caches at the ends of what fp32 arithmetic can hold: what an infinity
-or a NaN in V makes of the output, in every form of the launch.  Reference: the same attention in
-fp64."""
+"""Decode attention of 16-bit caches at the ends of what fp32 arithmetic can hold, in every form of the
+launch: infinities and NaN in V, the rounding of long sums.  Reference: the same attention in fp64."""
 import math
 
 import pytest
@@ -92,3 +91,41 @@ def test_infinities_in_v(native_libs, dtype, form):
     assert torch.equal(torch.where(ref.isinf(), got, 0.), torch.where(ref.isinf(), ref, 0.))
     finite = ref.isfinite()
     kvtest.assert_attention_close(got[finite].float().cpu().numpy(), ref[finite].float().cpu().numpy(), f"{dtype} {form}", dtype)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("entry", ["paged_decode", "paged_decode_overlapped"])
+def test_long_sums_are_rounded_not_cut_off(native_libs, dtype, entry):
+    """V of two neighbouring values in about equal shares: outputs near the middle between the two show
+    to which side their sums err.  Two hundred tiles a warp, each cut off by half of 2^-24 on
+    average, would take 6e-6 off; sums rounded to nearest err by sqrt(200) * 2^-25 or so."""
+    import torch
+    from orinmllm_b200 import capi
+    dt = kvtest.torch_dtype(dtype)
+    h, kv, n, batch = 32, 8, 32768, 16
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    step = 2.0 ** (-10 if dtype == "f16" else -7)
+    kp = torch.randn(n // 16, kv, 16, 128, generator=gen, device="cuda").to(dt)
+    vp = (1 + step * (torch.rand(n // 16, kv, 16, 128, generator=gen, device="cuda") < 0.5)).to(dt)
+    table = torch.arange(n // 16, dtype=torch.int32, device="cuda").expand(batch, -1).contiguous()  # all share their blocks
+    q = (torch.randn(batch, h * 128, generator=gen, device="cuda") * 0.2).to(dt)
+    out = torch.empty_like(q)
+    lay = capi.layout_paged(capi.dtype_code(dt), kv, 128, 16, n // 16)
+    nbytes = capi.decode_workspace_bytes(batch, h, kv)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    capi.workspace_init(ws, nbytes)
+    lens = torch.full((batch,), n, dtype=torch.int32, device="cuda")
+    getattr(capi, entry)(out, q, kp, vp, lay, table, n // 16, lens, 0, batch, h, 1 / math.sqrt(128), ws, nbytes)
+    k, v = (x.transpose(1, 2).reshape(n, kv, 128) for x in (kp, vp))
+    told = 0
+    for b in (0, 7, 15):
+        ref = torch.cat([torch.softmax(q[b].view(kv, 4, 128)[j].double() @ k[:, j].double().T / math.sqrt(128), -1) @ v[:, j].double()
+                         for j in range(kv)])
+        from_middle = ref - (1 + step / 2)
+        clear = from_middle.abs() > 2e-6
+        got = out[b].view(h, 128).double()
+        want = torch.where(from_middle > 0, 1 + step, 1.0)
+        wrong = clear & (got != want)
+        told += (clear & (from_middle.abs() < 5e-6)).sum().item()
+        assert not wrong.any(), f"{dtype} {entry}: {wrong.sum().item()} of {clear.sum().item()} fell to the wrong side"
+    assert told > 100  # outputs close enough to the middle to tell
