@@ -9,7 +9,10 @@
 //   scores:  rows 0..7 = the eight query heads, rows 8..15 zero;
 //   output:  rows 0..7 = P_hi, rows 8..15 = P_lo of the same heads, p = P_hi + P_lo in two 16-bit
 //            terms, so that the second term costs no instruction of its own; the two row halves of
-//            the fp32 accumulator are added once, when the item ends.
+//            the fp32 accumulator are added once, when the item ends.  Two bf16 terms hold 16 bits of
+//            a weight and not the 24 it has: bf16 caches take a second product with half of P_hi in
+//            both and a third term P_lo2 in its rows 8..15 (no row of a product is left at 0, which
+//            times an infinity in V would be NaN).
 // Thread (g = lane / 4, t = lane % 4) holds head g and tokens 2t, 2t+1, 2t+8, 2t+9 of the scores:
 // the layout of the accumulator is that of the A operand of the second product, so weights never
 // leave their thread; the row maximum is two shuffles.  Q enters unscaled, exactly as stored; the
@@ -56,6 +59,7 @@ template <typename T>
 struct Mma;
 template <>
 struct Mma<__half> {
+  static constexpr int kTerms = 2;            // 16-bit terms that hold a weight: 22 bits, the accuracy of ex2.approx
   static constexpr float kWeightBias = 12.f;  // log2 of the scale the weights carry
   static __device__ __forceinline__ void run(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                              uint32_t b0, uint32_t b1) {
@@ -74,6 +78,7 @@ struct Mma<__half> {
 };
 template <>
 struct Mma<__nv_bfloat16> {
+  static constexpr int kTerms = 3;  // (two would hold 16 bits)
   static constexpr float kWeightBias = 0.f;
   static __device__ __forceinline__ void run(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                              uint32_t b0, uint32_t b1) {
@@ -105,7 +110,7 @@ struct MmaTile {
   uint32_t qa[8][2];  // A fragments: k step s holds d = 16s + 2t, +1 and 16s + 8 + 2t, +1 of head g
   float acc[16][4];   // d = 8 * tile + 2t, +1 of head g: [0..1] the P_hi part, [2..3] the P_lo part
   float m, l;         // of head g; l: of the thread's own tokens until finish()
-  uint32_t hi[2], lo[2];  // weights of the block whose output pass comes next
+  uint32_t hi[2], lo[2], lo2[2];  // weights of the block whose output pass comes next (lo2: kTerms == 3)
   int g, t;               // head; position in the quad
   // ldmatrix addresses: lane 8m + r names row r of matrix m.  K: matrix m = 16-byte chunk m (mod 4)
   // of tokens r; V: matrix m = tokens (m & 1) * 8 + r, chunk m >> 1 (mod 2).
@@ -178,15 +183,21 @@ struct MmaTile {
     for (int e = 0; e < 4; ++e) {
       w[e] = fast_exp2(s[e] - m_new + M::kWeightBias);
       if (kTail && token(e) >= nvalid) w[e] = 0.f;
-      // 0 only where the weight is (see finish()); a bf16 value reaches as low as a weight does
-      first[e] = std::is_same<T, __half>::value && w[e] > 0.f ? fmaxf(w[e], kLeastHalf) : w[e];
+      // 0 only where the weight is (see finish())
+      first[e] = M::kTerms == 3 ? 0.5f * w[e] : (w[e] > 0.f ? fmaxf(w[e], kLeastHalf) : 0.f);
     }
     l = l * alpha + ((w[0] + w[1]) + (w[2] + w[3]));
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       hi[h] = M::pack(first[2 * h], first[2 * h + 1]);
       const float2 f = M::unpack(hi[h]);
-      lo[h] = M::pack(w[2 * h] - f.x, w[2 * h + 1] - f.y);
+      float2 r = make_float2(w[2 * h] - f.x, w[2 * h + 1] - f.y);
+      if constexpr (M::kTerms == 3) r = make_float2(r.x - f.x, r.y - f.y);
+      lo[h] = M::pack(r.x, r.y);
+      if constexpr (M::kTerms == 3) {
+        const float2 f2 = M::unpack(lo[h]);
+        lo2[h] = M::pack(r.x - f2.x, r.y - f2.y);
+      }
     }
     if (__any_sync(0xffffffffu, changed)) {
 #pragma unroll
@@ -220,6 +231,10 @@ struct MmaTile {
       float d[2][4] = {};
 #pragma unroll
       for (int u = 0; u < 2; ++u) M::run(d[u], hi[0], lo[0], hi[1], lo[1], b[2 * u], b[2 * u + 1]);
+      if (M::kTerms == 3) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) M::run(d[u], hi[0], lo2[0], hi[1], lo2[1], b[2 * u], b[2 * u + 1]);
+      }
 #pragma unroll
       for (int u = 0; u < 2; ++u)
 #pragma unroll

@@ -1,5 +1,6 @@
 """Decode attention of 16-bit caches at the ends of what fp32 arithmetic can hold, in every form of the
-launch: infinities and NaN in V, the rounding of long sums.  Reference: the same attention in fp64."""
+launch: infinities and NaN in V, the last bits of the weights, the rounding of long sums.  Reference:
+the same attention in fp64."""
 import math
 
 import pytest
@@ -91,6 +92,38 @@ def test_infinities_in_v(native_libs, dtype, form):
     assert torch.equal(torch.where(ref.isinf(), got, 0.), torch.where(ref.isinf(), ref, 0.))
     finite = ref.isfinite()
     kvtest.assert_attention_close(got[finite].float().cpu().numpy(), ref[finite].float().cpu().numpy(), f"{dtype} {form}", dtype)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("form", FORMS)
+def test_weights_keep_their_bits(native_libs, dtype, form):
+    """Three tokens of weights 1, 1 and w, and V such that the output is what is left of w beyond the
+    two 16-bit terms nearest to it: 2^-17 of w for bf16.  Bound: ex2.approx errs by 2^-22, the score
+    and three roundings of the sums by 2^-24 each, against a sum of weights of at least 2."""
+    import torch
+    dt = kvtest.torch_dtype(dtype)
+    n, (h, kv) = FORMS[form][2:]
+    mul = h // kv
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    q = torch.zeros(h, 128, device="cuda", dtype=dt)
+    q[:, 0] = (0.2 + 5 * torch.rand(h, generator=gen, device="cuda")).to(dt)
+    q[:, 1] = 1
+    k = torch.zeros(n, kv, 128, device="cuda", dtype=dt)
+    k[:, :, 1] = -4000  # weight 0
+    at = [n // 32 * 16 + i for i in range(3)]  # (of one block: what is cut apart is added up in fp32)
+    k[at, :, 1] = 0
+    k[at[2], :, 0] = -1
+    scale = 0.125
+    w = torch.exp(-q[:, 0].double() * scale)
+    first = w.to(dt)
+    second = (w - first.double()).to(dt)
+    v = torch.randn(n, kv, 128, generator=gen, device="cuda").to(dt)
+    heads = torch.arange(h, device="cuda")
+    j, d = heads // mul, heads % mul  # head d of KV head j looks at dimension d
+    v[at[0], j, d], v[at[1], j, d], v[at[2], j, d] = -first, -second, 1
+    got, ref = decode(form, q, k, v, scale).double(), reference(q, k, v, scale)
+    err = (got - ref)[heads, d].abs().max().item()
+    assert err <= (2.0 ** -22 + 4 * 2.0 ** -24) / 2, f"{dtype} {form}: {err:.2e}"
 
 
 @pytest.mark.parametrize("dtype", ["f16", "bf16"])
