@@ -111,7 +111,7 @@ struct FmaTile {
     return r;
   }
   float w[4][QH];
-  __device__ __forceinline__ void scores(const uint8_t* kt, int nvalid, bool, float) {
+  __device__ __forceinline__ void scores(const uint8_t* kt, int nvalid, bool) {
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       float2 f[8];
@@ -168,7 +168,7 @@ struct FmaTile {
     }
   }
   // after finish(): one more token whose rows are at k_row and v_row
-  __device__ __forceinline__ void add_token(const uint8_t* k_row, const uint8_t* v_row, float) {
+  __device__ __forceinline__ void add_token(const uint8_t* k_row, const uint8_t* v_row) {
     float2 kf[8], vf[8];
     row16(k_row, sub, kf);
     row16(v_row, sub, vf);
@@ -341,7 +341,7 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
     const bool linear = rows < kBS && !p.tile_contig;
     ok = wait_tile(bars + i % NS, phase);
     if (!ok) break;
-    tile.scores(ring + (i % NS) * C::kTileB, rows, linear, p.qscale);
+    tile.scores(ring + (i % NS) * C::kTileB, rows, linear);
     ok = wait_tile(bars + NS + i % NS, phase);
     if (!ok) break;
     tile.output(ring + (NS + i % NS) * C::kTileB, rows, linear);
@@ -356,7 +356,7 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
     if (takes_token) {
       const uint8_t* k_row = stage + QH * Tile::kRowStride;
       const uint8_t* v_row = k_row + Tile::kRowStride;
-      tile.add_token(k_row, v_row, p.qscale);
+      tile.add_token(k_row, v_row);
       if (hg == 0) {
         const int id = *reinterpret_cast<const int32_t*>(stage + (QH + 2) * Tile::kRowStride);
         if (id < 0 || (p.num_blocks > 0 && id >= p.num_blocks)) {

@@ -15,8 +15,8 @@
 //            times an infinity in V would be NaN).
 // Thread (g = lane / 4, t = lane % 4) holds head g and tokens 2t, 2t+1, 2t+8, 2t+9 of the scores:
 // the layout of the accumulator is that of the A operand of the second product, so weights never
-// leave their thread; the row maximum is two shuffles.  Q enters unscaled, exactly as stored; the
-// softmax scale is applied to the fp32 scores.  The weights of fp16 caches are scaled by 2^12 (the
+// leave their thread; the row maximum is two shuffles.  Q enters exactly as stored (bf16
+// rows times a power of two, Mma::row_scale); the softmax scale is applied to the fp32 scores.  The weights of fp16 caches are scaled by 2^12 (the
 // running sum with them), which keeps P_lo of small weights out of the subnormals.
 //
 // Tiles arrive by TMA through 128-byte-swizzled tensor maps of the pools ([half row][16 tokens][64
@@ -68,6 +68,8 @@ struct Mma<__half> {
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
   }
+  // the part of the softmax scale that the scores take; products of fp16 rows fit fp32 as they are
+  static __device__ __forceinline__ float score_scale(float qscale) { return qscale; }
   static __device__ __forceinline__ uint32_t pack(float x, float y) {
     const __half2 h = __floats2half2_rn(x, y);
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -86,6 +88,15 @@ struct Mma<__nv_bfloat16> {
         "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  }
+  // bf16 rows reach as far as fp32 does, and their products beyond it although the scaled score need not:
+  // the rows take the power of two of the scale, which is exact, the scores its mantissa
+  static __device__ __forceinline__ bool normal(float qscale) { return (__float_as_uint(qscale) & 0x7f800000u) != 0; }
+  static __device__ __forceinline__ float row_scale(float qscale) {
+    return normal(qscale) ? __uint_as_float(__float_as_uint(qscale) & 0x7f800000u) : 1.f;
+  }
+  static __device__ __forceinline__ float score_scale(float qscale) {
+    return normal(qscale) ? __uint_as_float((__float_as_uint(qscale) & 0x807fffffu) | 0x3f800000u) : qscale;
   }
   static __device__ __forceinline__ uint32_t pack(float x, float y) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
@@ -107,6 +118,7 @@ struct MmaTile {
   // at a time over the banks
   static constexpr int kRowStride = kRowB + 16;
   static constexpr bool kTensorMaps = true;
+  float by;           // what a product with the query rows is multiplied by to be a score (set by load_q)
   uint32_t qa[8][2];  // A fragments: k step s holds d = 16s + 2t, +1 and 16s + 8 + 2t, +1 of head g
   float acc[16][4];   // d = 8 * tile + 2t, +1 of head g: [0..1] the P_hi part, [2..3] the P_lo part
   float m, l;         // of head g; l: of the thread's own tokens until finish()
@@ -135,7 +147,7 @@ struct MmaTile {
     reset();
   }
   // rows of the group's heads, `stride` bytes apart; heads from `heads` on are zero
-  __device__ __forceinline__ void load_q(const uint8_t* rows, int stride, int heads, float) {
+  __device__ __forceinline__ void load_q(const uint8_t* rows, int stride, int heads, float qscale) {
     const bool valid = g < heads;
     const uint32_t* qh = reinterpret_cast<const uint32_t*>(rows + (valid ? g : 0) * stride) + t;
 #pragma unroll
@@ -143,12 +155,23 @@ struct MmaTile {
       qa[s][0] = valid ? qh[8 * s] : 0u;
       qa[s][1] = valid ? qh[8 * s + 4] : 0u;
     }
+    by = M::score_scale(qscale);
+    if constexpr (std::is_same<T, __nv_bfloat16>::value) {
+      const float rows_by = M::row_scale(qscale);
+#pragma unroll
+      for (int s = 0; s < 8; ++s)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const float2 f = M::unpack(qa[s][h]);
+          qa[s][h] = M::pack(f.x * rows_by, f.y * rows_by);
+        }
+    }
   }
   __device__ __forceinline__ int token(int e) const { return 2 * t + (e & 1) + (e >> 1) * 8; }
   // Scores and weights of the block whose K tile is at kt; kTail: only nvalid of its tokens exist
   // (linear: its rows lie one after the other, not swizzled).
   template <bool kTail>
-  __device__ __forceinline__ void scores_of(uint32_t kt, int nvalid, bool linear, float qscale) {
+  __device__ __forceinline__ void scores_of(uint32_t kt, int nvalid, bool linear) {
     float c0[4] = {0.f, 0.f, 0.f, 0.f}, c1[4] = {0.f, 0.f, 0.f, 0.f};  // tokens 0..7, 8..15
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -165,7 +188,7 @@ struct MmaTile {
       M::run(c0, qa[2 * i + 1][0], 0u, qa[2 * i + 1][1], 0u, b0[2], b0[3]);
       M::run(c1, qa[2 * i + 1][0], 0u, qa[2 * i + 1][1], 0u, b1[2], b1[3]);
     }
-    float s[4] = {c0[0] * qscale, c0[1] * qscale, c1[0] * qscale, c1[1] * qscale};
+    float s[4] = {c0[0] * by, c0[1] * by, c1[0] * by, c1[1] * by};
     if (kTail) {
 #pragma unroll
       for (int e = 0; e < 4; ++e)
@@ -246,9 +269,9 @@ struct MmaTile {
         }
     }
   }
-  __device__ __forceinline__ void scores(const uint8_t* kt, int nvalid, bool linear, float qscale) {
-    if (nvalid < kBS) scores_of<true>(smem_u32(kt), nvalid, linear, qscale);
-    else scores_of<false>(smem_u32(kt), nvalid, false, qscale);
+  __device__ __forceinline__ void scores(const uint8_t* kt, int nvalid, bool linear) {
+    if (nvalid < kBS) scores_of<true>(smem_u32(kt), nvalid, linear);
+    else scores_of<false>(smem_u32(kt), nvalid, false);
   }
   __device__ __forceinline__ void output(const uint8_t* vt, int nvalid, bool linear) {
     if (nvalid < kBS) output_of<true>(smem_u32(vt), nvalid, linear);
@@ -269,7 +292,7 @@ struct MmaTile {
         if (fabsf(acc[i][2 + e]) < INFINITY) acc[i][e] += acc[i][2 + e];
   }
   // after finish(): one more token whose rows are at k_row and v_row
-  __device__ __forceinline__ void add_token(const uint8_t* k_row, const uint8_t* v_row, float qscale) {
+  __device__ __forceinline__ void add_token(const uint8_t* k_row, const uint8_t* v_row) {
     const uint32_t* kr = reinterpret_cast<const uint32_t*>(k_row) + t;
     const uint32_t* vr = reinterpret_cast<const uint32_t*>(v_row) + t;
     float s = 0.f;
@@ -282,7 +305,7 @@ struct MmaTile {
       }
     s += __shfl_xor_sync(0xffffffffu, s, 1);
     s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s *= qscale;
+    s *= by;
     const float m_new = fmaxf(m, s);
     const float a = fast_exp2(m - m_new), w = fast_exp2(s - m_new + M::kWeightBias);
     m = m_new;
@@ -511,7 +534,7 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
     if (kFused && has_item_end) {
       // Fused step: this piece ends the item, so it also carries the new token (position
       // item.len, not in the pool yet), staged when the item began.
-      tile.add_token(stage + kMmaHeads * C::kRowStride, stage + (kMmaHeads + 1) * C::kRowStride, p.qscale);
+      tile.add_token(stage + kMmaHeads * C::kRowStride, stage + (kMmaHeads + 1) * C::kRowStride);
       // append: the first head group's warp stores the rows (lanes 0..15 the K row, 16..31 the V
       // row) into the block that holds position item.len
       if (hg == 0) {
@@ -668,7 +691,7 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
     constexpr bool kTail = decltype(tail_tag)::value;
     const bool linear = kTail && !p.tile_contig;  // rows copied one by one, not swizzled
     if (!wait_slot(bars + slot, phase)) return false;
-    tile.template scores_of<kTail>(ring_u + slot * C::kTileB, nvalid, linear, p.qscale);
+    tile.template scores_of<kTail>(ring_u + slot * C::kTileB, nvalid, linear);
     __syncwarp();  // the K slot is read
     if (k_issued < n) {
       if (lane == 0) fence_proxy_async();

@@ -1,6 +1,6 @@
 """Decode attention of 16-bit caches at the ends of what fp32 arithmetic can hold, in every form of the
-launch: infinities and NaN in V, the last bits of the weights, the rounding of long sums.  Reference:
-the same attention in fp64."""
+launch: infinities and NaN in V, the last bits of the weights, the rounding of long sums, products
+beyond 2^128.  Reference: the same attention in fp64."""
 import math
 
 import pytest
@@ -162,3 +162,22 @@ def test_long_sums_are_rounded_not_cut_off(native_libs, dtype, entry):
         told += (clear & (from_middle.abs() < 5e-6)).sum().item()
         assert not wrong.any(), f"{dtype} {entry}: {wrong.sum().item()} of {clear.sum().item()} fell to the wrong side"
     assert told > 100  # outputs close enough to the middle to tell
+
+
+@pytest.mark.parametrize("dtype", ["f16", "bf16"])
+@pytest.mark.parametrize("form", FORMS)
+def test_products_beyond_fp32_before_the_scale(native_libs, dtype, form):
+    """bf16 rows may be so large that q . k passes 2^128 while the scaled score does not."""
+    import torch
+    dt = kvtest.torch_dtype(dtype)
+    n, (h, kv) = FORMS[form][2:]
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    big = 2.0 ** 63 if dtype == "bf16" else 2.0 ** 15
+    q = torch.zeros(h, 128, device="cuda", dtype=dt)
+    q[:, :8] = big
+    k = torch.zeros(n, kv, 128, device="cuda", dtype=dt)
+    k[:, :, :8] = (big * (0.5 + 0.5 * torch.rand(n, kv, 8, generator=gen, device="cuda"))).to(dt)
+    v = torch.randn(n, kv, 128, generator=gen, device="cuda").to(dt)
+    scale = 2.0 ** -126 if dtype == "bf16" else 2.0 ** -30
+    got, ref = decode(form, q, k, v, scale), reference(q, k, v, scale)
+    kvtest.assert_attention_close(got.float().cpu().numpy(), ref.float().cpu().numpy(), f"{dtype} {form}", dtype)
