@@ -1072,7 +1072,8 @@ constexpr int kMinPartialSlots = 2 * kMaxSms * kMaxWarpsPerCta;  // two per warp
 constexpr int kStatusBytes = 256;
 // Floats of a workspace slot of `heads` heads; the counters of the two-level assembly live in the
 // last slot of an area of kMinPartialSlots slots of heads_per_warp(kv_mul) heads.
-constexpr int slot_floats_of(int heads) { return heads * kD + 8; }
+// (eight heads take two slots of four)
+constexpr int slot_floats_of(int heads) { return heads > 4 ? 2 * slot_floats_of(4) : heads * kD + 8; }
 
 // Tuning knob: 0 = default shape; set through kpx_internal_set_decode_variant.
 extern int g_decode_variant;

@@ -350,6 +350,76 @@ struct MmaCfg {
   static_assert(kWarpRingB % 1024 == 0 && kOffStage % 16 == 0, "alignment of the slots and of the staging area");
 };
 
+// Adds up the pieces of an item in `cnt` workspace slots of SH heads (the first is slot `first`, the
+// i-th one after it slot from + 2 i): into one unnormalised slot at dst, or into the item's output
+// rows if dst is nullptr.  32 / SH lanes share a head, so that all lanes have loads in flight however
+// few heads there are.  One pass: the maxima, sums and accumulators of kBatch slots are requested
+// together and folded into the running ones, so that a batch is one trip to L2.  us per launch in a
+// graph, four lanes a head whatever their number and three passes over the slots -> this; fp16:
+// 8/8 heads, one sequence of 2000 tokens in the line of blocks 29.0 -> 17.6, 8 of 64..800 28.0 -> 17.0,
+// 32/8, one of 2000 23.2 -> 15.9, one of 131072 104.5 -> 96.8 (and 238 registers a thread, not 255).
+template <typename T, int SH>
+__device__ __forceinline__ void merge_slots(const float* slots, int64_t first, int64_t from, int cnt, int heads,
+                                            float* dst, T* rows, int lane) {
+  constexpr int kLanes = 32 / SH, kVecs = kD / 4 / kLanes, kBatch = kVecs > 2 ? 16 / kVecs : 8;
+  constexpr int64_t kFloats = slot_floats_of(SH);
+  const int head = lane / kLanes, t = lane % kLanes;
+  if (head >= heads) return;
+  const float* row = slots + head * kD + 4 * t;
+  const float* stats = slots + SH * kD + head;
+  float m = -INFINITY, l = 0.f;
+  float4 o[kVecs];
+#pragma unroll
+  for (int k = 0; k < kVecs; ++k) o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (int i0 = 0; i0 < cnt; i0 += kBatch) {
+    float mi[kBatch], li[kBatch], m_new = m;
+    float4 v[kBatch][kVecs];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int i = min(i0 + u, cnt - 1);
+      const int64_t at = (i ? from + 2 * i : first) * kFloats;
+      mi[u] = i0 + u < cnt ? __ldcg(stats + at) : -INFINITY;  // (a slot read twice has no weight)
+      li[u] = __ldcg(stats + at + SH);
+#pragma unroll
+      for (int k = 0; k < kVecs; ++k) v[u][k] = __ldcg(reinterpret_cast<const float4*>(row + at + 4 * k * kLanes));
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) m_new = fmaxf(m_new, mi[u]);
+    const float a = fast_exp2(m - m_new);
+    m = m_new;
+    l *= a;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k) o[k] = make_float4(o[k].x * a, o[k].y * a, o[k].z * a, o[k].w * a);
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (i0 + u >= cnt) break;
+      const float w = fast_exp2(mi[u] - m);
+      l = fmaf(li[u], w, l);
+#pragma unroll
+      for (int k = 0; k < kVecs; ++k) {
+        o[k].x = fmaf(v[u][k].x, w, o[k].x);
+        o[k].y = fmaf(v[u][k].y, w, o[k].y);
+        o[k].z = fmaf(v[u][k].z, w, o[k].z);
+        o[k].w = fmaf(v[u][k].w, w, o[k].w);
+      }
+    }
+  }
+  if (dst) {
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k) *reinterpret_cast<float4*>(dst + head * kD + 4 * (k * kLanes + t)) = o[k];
+    if (t == 0) {
+      dst[SH * kD + head] = m;
+      dst[SH * kD + SH + head] = l;
+    }
+  } else {
+    const float inv = 1.f / l;
+#pragma unroll
+    for (int k = 0; k < kVecs; ++k)
+      MmaTile<T>::write4(rows + head * kD, 4 * (k * kLanes + t),
+                         make_float4(o[k].x * inv, o[k].y * inv, o[k].z * inv, o[k].w * inv));
+  }
+}
+
 template <typename T, int NW, int NS, int CPS, bool kFused>
 __global__ void __launch_bounds__(32 * NW, CPS)
 paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap map_k,
@@ -561,7 +631,7 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
     }
     // one workspace slot: slot_heads accumulators of 128, then their maxima, then their sums
     const int sh = p.slot_heads;
-    const int64_t slot_floats = sh > 4 ? 2 * slot_floats_of(4) : slot_floats_of(sh);
+    const int64_t slot_floats = slot_floats_of(sh);
     if (head_ok) tile.store(p.partials + partial_slot * slot_floats, sh);
     // The item is cut by a range boundary.  Publish this piece, then count it; the warp
     // that brings the count up to the number of pieces assembles the item from all of
@@ -582,59 +652,6 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
       __syncwarp();
       return true;
     };
-    auto slot_of = [&](int64_t c) -> const float* {  // only the first piece can be a "tail" slot
-      return p.partials + ((c == c_first) ? 2 * c + 1 : 2 * c) * slot_floats;
-    };
-    // Merges cnt slots into the item's output rows (dst == nullptr) or into one unnormalised slot:
-    // the quad of head g handles that head, thread t the dims 16k + 4t, +1, +2, +3.  The weights
-    // 2^(m_c - max) need the overall maximum first; with it every slot's term is independent, so
-    // the loads of the accumulation loop can be in flight together.
-    auto merge = [&](int cnt, auto slot_fn, float* dst) {
-      float mx = -INFINITY, sum = 0.f;
-      if (head_ok)
-        for (int i = t; i < cnt; i += 4) mx = fmaxf(mx, __ldcg(slot_fn(i) + sh * kD + g));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-      if (head_ok)
-        for (int i = t; i < cnt; i += 4) {
-          const float* ps = slot_fn(i);
-          sum += __ldcg(ps + sh * kD + sh + g) * fast_exp2(__ldcg(ps + sh * kD + g) - mx);
-        }
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      if (!head_ok) return;
-      float4 o[8];
-#pragma unroll
-      for (int k = 0; k < 8; ++k) o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 2
-      for (int i = 0; i < cnt; ++i) {
-        const float* ps = slot_fn(i);
-        const float w = fast_exp2(__ldcg(ps + sh * kD + g) - mx);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const float4 v = __ldcg(reinterpret_cast<const float4*>(ps + g * kD + 16 * k + 4 * t));
-          o[k].x = fmaf(v.x, w, o[k].x);
-          o[k].y = fmaf(v.y, w, o[k].y);
-          o[k].z = fmaf(v.z, w, o[k].z);
-          o[k].w = fmaf(v.w, w, o[k].w);
-        }
-      }
-      if (dst) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) *reinterpret_cast<float4*>(dst + g * kD + 16 * k + 4 * t) = o[k];
-        if (t == 0) {
-          dst[sh * kD + g] = mx;
-          dst[sh * kD + sh + g] = sum;
-        }
-      } else {
-        const float inv = 1.f / sum;
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-          *reinterpret_cast<uint2*>(orow + 16 * k + 4 * t) =
-              make_uint2(M::pack(o[k].x * inv, o[k].y * inv), M::pack(o[k].z * inv, o[k].w * inv));
-      }
-    };
-    int* item_cnt = p.counters + (item.b * (p.num_kv_heads * p.head_groups) + item.sub);
     // An item cut into many pieces (one very long sequence) is assembled in two levels so that
     // no single warp reads them all: the pieces of `group` consecutive warps are merged by the
     // last of them to arrive into one slot of a second area, and the last group to finish
@@ -645,25 +662,44 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
     const int64_t W_all = int64_t(gridDim.x) * NW;
     const int64_t n_groups = (W_all + group - 1) / group;
     const int64_t group_base = int64_t(p.partial_slots) - 1 - 2 * n_groups;  // first group slot
-    if (pieces <= group || group_base < 2 * W_all || 2 * n_groups > slot_floats_of(sh > 4 ? 4 : sh)) {
-      if (arrive_last(item_cnt, pieces)) merge(pieces, [&](int i) { return slot_of(c_first + i); }, nullptr);
-      return;
+    const bool flat = pieces <= group || group_base < 2 * W_all || 2 * n_groups > slot_floats_of(sh > 4 ? 4 : sh);
+    // what is merged next: cnt slots (only an item's first piece can be a "tail" slot), and where to
+    int* counter = p.counters + (item.b * (p.num_kv_heads * p.head_groups) + item.sub);
+    int cnt = pieces;
+    int64_t first = 2 * c_first + 1, from = 2 * c_first;
+    float* dst = nullptr;
+    if (!flat) {
+      // A group holds pieces of at most two such items: one that entered it from the left (0) and
+      // one that starts inside it (1).
+      const int64_t gr = worker / group;
+      const int in = c_first < gr * group ? 0 : 1;
+      const int64_t g_lo = in ? c_first : gr * group;
+      const int64_t g_hi = c_last < gr * group + group - 1 ? c_last : gr * group + group - 1;
+      counter = p.group_counters + 2 * gr + in;
+      cnt = int(g_hi - g_lo) + 1;
+      first = 2 * g_lo + in;
+      from = 2 * g_lo;
+      dst = p.partials + (group_base + 2 * gr + in) * slot_floats;
     }
-    // A group holds pieces of at most two such items: one that entered it from the left (0) and
-    // one that starts inside it (1).
-    auto group_slot = [&](int64_t gr) {
-      return p.partials + (group_base + 2 * gr + ((c_first < gr * group) ? 0 : 1)) * slot_floats;
-    };
-    const int64_t gr = worker / group;
-    const int64_t g_lo = c_first > gr * group ? c_first : gr * group;
-    const int64_t g_hi = c_last < gr * group + group - 1 ? c_last : gr * group + group - 1;
-    int* group_cnt = p.group_counters + 2 * gr + ((c_first < gr * group) ? 0 : 1);
-    if (!arrive_last(group_cnt, int(g_hi - g_lo) + 1)) return;
-    merge(int(g_hi - g_lo) + 1, [&](int i) { return slot_of(g_lo + i); }, group_slot(gr));
-    __syncwarp();  // every lane's part of the group slot is ordered before lane 0's release
-    const int64_t G0 = c_first / group, G1 = c_last / group;
-    if (arrive_last(item_cnt, int(G1 - G0) + 1))
-      merge(int(G1 - G0) + 1, [&](int i) { return static_cast<const float*>(group_slot(G0 + i)); }, nullptr);
+    T* rows = static_cast<T*>(p.out) + (int64_t(item.b) * p.num_q_heads + item.kvh * p.kv_mul + hg * kMmaHeads) * kD;
+    const int heads = min(kMmaHeads, p.kv_mul - hg * kMmaHeads);
+    for (;;) {
+      if (!arrive_last(counter, cnt)) return;
+      switch (sh) {
+        case 1: merge_slots<T, 1>(p.partials, first, from, cnt, heads, dst, rows, lane); break;
+        case 2: merge_slots<T, 2>(p.partials, first, from, cnt, heads, dst, rows, lane); break;
+        case 4: merge_slots<T, 4>(p.partials, first, from, cnt, heads, dst, rows, lane); break;
+        default: merge_slots<T, kMmaHeads>(p.partials, first, from, cnt, heads, dst, rows, lane); break;
+      }
+      if (!dst) return;
+      __syncwarp();  // every lane's part of the group slot is ordered before lane 0's release
+      const int64_t G0 = c_first / group, G1 = c_last / group;
+      counter = p.counters + (item.b * (p.num_kv_heads * p.head_groups) + item.sub);
+      cnt = int(G1 - G0) + 1;
+      from = group_base + 2 * G0;
+      first = from + 1;  // (the item starts inside its first group)
+      dst = nullptr;
+    }
   };
 
   auto wait_slot = [&](uint64_t* bar, uint32_t ph) -> bool {
