@@ -76,7 +76,12 @@ int decode_rows(void* out, const void* q, const void* k_pool, const void* v_pool
 // runs then lies under the predecessor's end.  Every thread of such a kernel calls grid_wait()
 // before its first access to global memory, which returns when everything earlier on the stream
 // has completed and is visible; then grid_release() lets the successor's CTAs come.  A kernel so
-// launched behind any other work (a copy, somebody else's kernel) starts when that has ended.
+// launched behind any other work (a copy, somebody else's kernel) starts when that has ended, and a
+// successor whose CTAs do not fit beside this kernel's comes up as those leave.  The kernels that
+// run along the line of blocks fill their SMs and leave grid_release() out, which holds the successor
+// back until they end.  Measured with it -> without, us: fp32 12/2 heads, 200 short sequences, fused
+// 36.7 -> 34.3, one of 24000 tokens 31.6 -> 30.3; fp16 32/8, one of 131072 97.2 -> 95.4; bf16 28/4, a
+// step of 4 layers of 64 sequences 250 -> 245.
 // grid_wait() returns a zero the compiler cannot see through: added to a pointer that is read by
 // __ldg or declared __restrict__, it keeps such loads, which the compiler may otherwise move
 // across a memory clobber, behind the wait.

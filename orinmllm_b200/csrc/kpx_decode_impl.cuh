@@ -346,7 +346,7 @@ paged_decode_kernel(const DecodeParams p) {
     mbar_fence_init();
   }
   const int64_t after_wait = grid_wait();
-  if (CPS == 1) grid_release();  // (launches that overlap others leave the SMs to those)
+  // (no grid_release(): kpx_common.cuh)
   // With a plan of the step the prefix and this warp's starting point come from it: one round
   // trip to global memory instead of lengths -> prefix -> search -> first block id.
   bool planned = false;
