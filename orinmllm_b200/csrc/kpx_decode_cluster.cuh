@@ -534,7 +534,7 @@ int dispatch_decode_mma(DecodeParams p, cudaStream_t stream, int flags) {
   // at a time while the previous launch's last warps finish.
   const bool overlapped = (g_decode_variant & 3) == 1 ? true : ((g_decode_variant & 3) == 2 ? false : (flags & KPX_DECODE_OVERLAPPED) != 0);
   const bool small_ctas = overlapped && !p.small;
-  if (p.k_new) return small_ctas ? launch_mma_form<T, 4, 3, 2, true>(p, stream) : launch_mma_form<T, 8, 3, 1, true>(p, stream);
+  if (p.k_new) return small_ctas ? launch_mma_form<T, 4, 3, 2, true>(p, stream) : launch_mma_form<T, 8, 1, 1, true>(p, stream);
   // (slots per warp: kpx_decode_mma.cuh; launches that overlap keep three, 36 layers on three chains:
   // 6667 GB/s, with two 6643, with one 6153)
   return small_ctas ? launch_mma_form<T, 4, 3, 2, false>(p, stream) : launch_mma_form<T, 8, 1, 1, false>(p, stream);
