@@ -12,7 +12,7 @@ int g_decode_variant = 0;
 // is below g_small_below blocks per warp of the grid; then ranges hold at least
 // g_min_blocks_per_range blocks while at least g_min_warps_per_sm warps per SM stay active.
 int g_small_below = 12, g_min_blocks_per_range = 12, g_min_warps_per_sm = 4;
-int g_cluster_share = 24;
+int g_small_items = 4, g_cluster_share = 24;
 // Test-only: polls before a bounded wait gives up, and the warp whose first tile never comes.
 uint32_t g_wait_limit = kWaitLimit;
 int g_withhold_worker = -1;
@@ -30,6 +30,10 @@ extern "C" __attribute__((visibility("default"))) void kpx_internal_set_decode_s
   g_small_below = below;
   if (min_blocks > 0) g_min_blocks_per_range = min_blocks;
   if (min_warps >= 0) g_min_warps_per_sm = min_warps;
+}
+
+extern "C" __attribute__((visibility("default"))) void kpx_internal_set_decode_small_items(int below) {
+  g_small_items = below;
 }
 
 extern "C" __attribute__((visibility("default"))) void kpx_internal_set_decode_cluster(int max_share) {

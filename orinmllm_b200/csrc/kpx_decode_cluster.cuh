@@ -518,11 +518,16 @@ int try_cluster(const DecodeParams& p, int max_share, cudaStream_t stream) {
 template <typename T>
 int dispatch_decode_mma(DecodeParams p, cudaStream_t stream, int flags) {
   p.head_groups = (p.kv_mul + kMmaHeads - 1) / kMmaHeads;
-  p.small = small_launch(p, kMmaHeads, kMmaWarpsPerSm) ? 1 : 0;
+  const bool small = small_launch(p, kMmaHeads, kMmaWarpsPerSm);
+  // Fewer, longer ranges only where a launch is so few items that each would be cut into hundreds of
+  // pieces.  us per launch, cut so / as ever: one item of 60000 tokens (4/1 heads fp16) 29 / 38, two (16/2)
+  // 33 / 34, four of 40000..50000 39 / 36, 640 of 100..350 tokens (28/4 bf16) 27 / 23, 800 of 20..200
+  // (8/8 fp16) 23 / 18.
+  p.small = small && int64_t(p.batch) * p.num_kv_heads * p.head_groups < g_small_items ? 1 : 0;
   p.slot_heads = p.kv_mul > 4 ? kMmaHeads : heads_per_warp(p.kv_mul);
   // eight-head slots are twice a four-head slot
   if (p.slot_heads == kMmaHeads) p.partial_slots /= 2;
-  if (p.small && g_cluster_share > 0) {
+  if (small && g_cluster_share > 0) {
     // eight warps per item and SM, or four or two where there are more items than SMs
     int rc = try_cluster<MmaTile<T>, 8, 3>(p, g_cluster_share, stream);
     if (rc == KPX_ERR_UNIMPLEMENTED) rc = try_cluster<MmaTile<T>, 4, 3>(p, g_cluster_share, stream);
@@ -533,7 +538,7 @@ int dispatch_decode_mma(DecodeParams p, cudaStream_t stream, int flags) {
   // warps per SM instead of one of eight: an SM then takes up the next launch's work a half
   // at a time while the previous launch's last warps finish.
   const bool overlapped = (g_decode_variant & 3) == 1 ? true : ((g_decode_variant & 3) == 2 ? false : (flags & KPX_DECODE_OVERLAPPED) != 0);
-  const bool small_ctas = overlapped && !p.small;
+  const bool small_ctas = overlapped && !small;
   if (p.k_new) return small_ctas ? launch_mma_form<T, 4, 3, 2, true>(p, stream) : launch_mma_form<T, 8, 1, 1, true>(p, stream);
   // (slots per warp: kpx_decode_mma.cuh; launches that overlap keep three, 36 layers on three chains:
   // 6667 GB/s, with two 6643, with one 6153)

@@ -82,7 +82,7 @@ struct DecodeParams {
   // A plan of this step (nullptr: none), see the layout below: what every launch of the step
   // would otherwise work out again in its prologue.
   const int32_t* plan;
-  // 16-bit caches (kpx_decode_mma.cuh): few blocks per warp; heads a workspace slot holds; counters
+  // 16-bit caches (kpx_decode_mma.cuh): fewer, longer ranges; heads a workspace slot holds; counters
   // of the two-level assembly.
   int32_t small, slot_heads;
   int32_t* group_counters;
@@ -1081,6 +1081,8 @@ extern int g_decode_variant;
 // is below g_small_below blocks per warp of the grid; then ranges hold at least
 // g_min_blocks_per_range blocks while at least g_min_warps_per_sm warps per SM stay active.
 extern int g_small_below, g_min_blocks_per_range, g_min_warps_per_sm;
+// 16-bit caches: such ranges only for launches of fewer items than this.
+extern int g_small_items;
 // Most blocks a warp takes in the cluster form of a small launch (0: form off).
 extern int g_cluster_share;
 extern uint32_t g_wait_limit;
