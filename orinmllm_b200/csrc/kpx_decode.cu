@@ -94,17 +94,16 @@ constexpr int kPlanThreads = 128;
 // One thread per warp of the decode launch: where its range of the line of blocks starts.
 __global__ void __launch_bounds__(kPlanThreads) decode_plan_kernel(const DecodeParams p, int32_t* plan, int workers) {
   __shared__ int prefix[kMaxBatch + 1];
-  __shared__ int bad;
   const int tid = threadIdx.x;
   grid_wait();
   grid_release();
-  if (tid == 0) bad = 0;
+  int too_long = 0;  // a length that its table row cannot hold, seen by this thread
   for (int b = tid; b < p.batch; b += kPlanThreads) {
     prefix[b + 1] = blocks_of(seq_len_of(p, b));
-    if (p.block_table && p.seq_lens && p.seq_lens[b] + p.len_bias > p.max_cached_tokens) bad = 1;
+    if (p.block_table && p.seq_lens && p.seq_lens[b] + p.len_bias > p.max_cached_tokens) too_long = 1;
   }
   if (tid == 0) prefix[0] = 0;
-  __syncthreads();
+  const int bad = __syncthreads_or(too_long);
   if (tid < 32) {  // inclusive scan in chunks of 32
     int carry = 0;
     for (int base = 0; base < p.batch; base += 32) {

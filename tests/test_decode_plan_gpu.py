@@ -133,3 +133,22 @@ def test_plan_argument_checks(native_libs):
         capi.decode_plan(plan, plan.numel(), lay, table, 4, lens, 0, 4, 30)  # heads do not divide
     with pytest.raises(capi.KpxError):
         capi.decode_plan(None, plan.numel(), lay, table, 4, lens, 0, 4, 32)
+
+
+@pytest.mark.parametrize("batch", [1, 33, 128, 500])
+def test_an_over_long_length_is_always_reported(native_libs, batch):
+    """One length that its table row cannot hold, at every position of the batch in turn (every thread of
+    the plan's CTA sees it once): the plan hands the error on each time, and none without it."""
+    import torch
+    from orinmllm_b200 import capi
+
+    width = 2
+    lay = capi.layout_paged(capi.KPX_F16, 2, 128, 16, batch * width)
+    table = torch.arange(batch * width, dtype=torch.int32, device="cuda").view(batch, width)
+    plans = torch.zeros(batch + 1, capi.decode_plan_bytes(), dtype=torch.uint8, device="cuda")
+    lens = torch.full((batch + 1, batch), 16 * width, dtype=torch.int32, device="cuda")
+    lens[torch.arange(batch), torch.arange(batch)] += 1
+    for i in range(batch + 1):
+        capi.decode_plan(plans[i], plans.shape[1], lay, table, width, lens[i], 0, batch, 8)
+    errors = plans[:, 16:20].contiguous().view(torch.int32)[:, 0].tolist()
+    assert errors == [capi.KPX_ERR_INVALID_ARGUMENT] * batch + [0]
