@@ -122,6 +122,8 @@ __global__ void rope_append_kernel(T* __restrict__ q, T* __restrict__ k, const T
   slot_mapping += slot_mapping ? after_wait : 0;
   sin_cache += after_wait;
   cos_cache += after_wait;
+  q_norm_w += q_norm_w ? after_wait : 0;
+  k_norm_w += k_norm_w ? after_wait : 0;
   constexpr int E = Elt<T>::kPer16B;
   const int hs = L.head_size;
   const int groups_per_head = hs / 2 / E;  // pair-groups per head

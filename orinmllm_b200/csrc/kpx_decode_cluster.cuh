@@ -316,8 +316,8 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
     if (n > 0 || takes_token) {
       stage_new_token<T, QH, Tile::kRowStride>(
           reinterpret_cast<const T*>(q_rows) - int64_t(hg) * QH * kD, hg, p.kv_mul,
-          static_cast<const T*>(p.k_new) + (int64_t(b) * p.num_kv_heads + kvh) * kD,
-          static_cast<const uint8_t*>(p.v_new) + (int64_t(b) * p.num_kv_heads + kvh) * kRowB, takes_token,
+          static_cast<const T*>(p.k_new) + (int64_t(b) * p.num_kv_heads + kvh) * kD + after_wait,
+          static_cast<const uint8_t*>(p.v_new) + (int64_t(b) * p.num_kv_heads + kvh) * kRowB + after_wait, takes_token,
           p.sin_cache + int64_t(len) * kD + after_wait, p.cos_cache + int64_t(len) * kD + after_wait,
           row ? row + len / kBS : nullptr, len / kBS, stage, lane);
       __syncwarp();

@@ -478,8 +478,10 @@ template <typename T>
 __global__ void __launch_bounds__(kD* kMergeRowLanes)
     prefill_merge_kernel(T* __restrict__ out, const float* __restrict__ partials, const MergeDesc* __restrict__ descs,
                          int num_q_heads) {
-  descs += grid_wait();
+  const int64_t after_wait = grid_wait();
   grid_release();
+  descs += after_wait;
+  partials += after_wait;
   const MergeDesc md = descs[blockIdx.x];
   const int d = threadIdx.x;
 #pragma unroll

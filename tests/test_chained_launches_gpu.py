@@ -79,3 +79,57 @@ def test_a_chain_of_steps_sees_what_came_before(native_libs, dtype, batch, ctx, 
     torch.cuda.synchronize()
     assert capi.workspace_status(ws) == 0
     assert torch.equal(outs, want) and torch.equal(kp, wkp) and torch.equal(vp, wvp)
+
+
+@pytest.mark.parametrize("dtype", ["f16", "f32"])
+def test_inputs_written_by_the_launch_before(native_libs, dtype):
+    """The norm weights of a rotation and the new rows of a fused step are written by the chained launch
+    right in front of it (an append whose "pool" they are), other values every time: the results are
+    those with a wait after every launch."""
+    import torch
+    from orinmllm_b200 import capi
+    h, kv, batch, steps = 8, 2, 3, 40
+    dt = kvtest.torch_dtype(dtype)
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    lay = capi.layout_paged(capi.dtype_code(dt), kv, 128, 16, 64)
+    rows = {t: capi.layout_contiguous(capi.dtype_code(t), 1, 128, 16, 0) for t in (dt, torch.float32)}
+    table = torch.randperm(64, generator=gen, device="cuda")[:batch * 16].to(torch.int32).view(batch, 16)
+    pos = torch.tensor([5, 100, 200], dtype=torch.int32, device="cuda")
+    at = torch.arange(batch, device="cuda")
+    slots = table[at, (pos // 16).long()].long() * 16 + pos % 16
+    sin, cos = (torch.empty(256 * 128, device="cuda") for _ in range(2))
+    capi.sin_cos_cache(sin, cos, 128, 256, 1e6)
+    weights = torch.rand(steps, 2, 128, generator=gen, device="cuda") + 0.5
+    fresh = torch.randn(steps, batch * (h + 2 * kv), 128, generator=gen, device="cuda").to(dt)
+    pools0 = [torch.randn(64, kv, 16, 128, generator=gen, device="cuda").to(dt) for _ in range(2)]
+    nbytes = capi.decode_workspace_bytes(batch, h, kv)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    capi.workspace_init(ws, nbytes)
+
+    def run(wait):
+        kp, vp = (p.clone() for p in pools0)
+        outs = torch.zeros(steps, batch, h * 128, device="cuda", dtype=dt)
+        w = torch.zeros(2, 128, device="cuda")
+        x = torch.zeros(batch * (h + 2 * kv), 128, device="cuda", dtype=dt)
+        q, k, v = x[:batch * h], x[batch * h:batch * (h + kv)], x[batch * (h + kv):]
+        torch.cuda.synchronize()
+        for i in range(steps):
+            capi.append(x, None, rows[dt], fresh[i], None, num_tokens=len(x))
+            wait()
+            if i % 2:
+                capi.rope_append_decode(outs[i], q, k, v, sin, cos, kp, vp, lay, table, 16, pos, batch, h, 1 / math.sqrt(128),
+                                        ws, nbytes)
+            else:
+                capi.append(w, None, rows[torch.float32], weights[i], None, num_tokens=2)
+                wait()
+                capi.norm_rope_append(q, k, v, h, w[0], w[1], 1e-6, pos, sin, cos, kp, vp, lay, slots, batch)
+                wait()
+                capi.append(outs[i].view(-1, 128), None, rows[dt], q, None, num_tokens=len(q))
+            wait()
+        torch.cuda.synchronize()
+        return outs, kp, vp
+
+    want = run(torch.cuda.synchronize)
+    for got, ref in zip(run(lambda: None), want):
+        assert torch.equal(got, ref)
+    assert capi.workspace_status(ws) == 0
