@@ -4,7 +4,7 @@ summarised under profiles/ were taken on.
 
     python tests/profiling/decode_case.py [launches] [large|overlapped]
 
-`overlapped` launches the three-small-CTAs-per-SM form (kpx_paged_decode_overlapped), `large`
+`overlapped` launches the two-small-CTAs-per-SM form (kpx_paged_decode_overlapped), `large`
 (default) the one-CTA-per-SM form (kpx_paged_decode).
 """
 import sys

@@ -146,6 +146,7 @@ def test_decode_placement_invariance(native_libs, oracle):
     assert torch.equal(outs[0], outs[1])
 
 
+@pytest.mark.parametrize("cluster", [24, 0], ids=["cluster_form", "line_of_blocks"])
 @pytest.mark.parametrize("knobs", [(0, 12, 4), (1 << 20, 20, 0), (1 << 20, 3, 1), (1 << 20, 12, 4)])
 @pytest.mark.parametrize("dtype,heads,lens", [
     ("f16", (32, 8), [4096]),                 # one sequence: every item is cut into many pieces
@@ -153,16 +154,20 @@ def test_decode_placement_invariance(native_libs, oracle):
     ("f32", (8, 8), [2000, 1]),
     ("f16", (4, 1), [40000]),                 # one KV head of one long sequence (the sharded case)
 ])
-def test_decode_small_launch_forms(native_libs, oracle, knobs, dtype, heads, lens):
-    """Launches with few blocks per warp run a form of the kernel that cuts the work into fewer,
-    longer ranges on CTA-minor warp numbers.  Whatever the cut (off; as coarse as 20 blocks per
-    range with idle SMs allowed; as fine as 3), outputs meet the oracle, twice in a row on the
-    same workspace."""
+def test_decode_small_launch_forms(native_libs, oracle, cluster, knobs, dtype, heads, lens):
+    """Launches with few blocks per warp run as one cluster of CTAs per item, or, where that is not
+    for them (here: switched off), in a form that cuts the line of blocks into fewer, longer ranges
+    on CTA-minor warp numbers.  Whatever the cut (off; as coarse as 20 blocks per range with idle
+    SMs allowed; as fine as 3), outputs meet the oracle, twice in a row on the same workspace."""
     from orinmllm_b200 import capi
     lib = capi.lib()
     try:
         lib.kpx_internal_set_decode_small(*knobs)
+        lib.kpx_internal_set_decode_cluster(cluster)
+        lib.kpx_internal_set_decode_small_items(1 << 20)
         case = kvtest.make_paged_case(29, dtype, heads[0], heads[1], lens)
         _run_case(oracle, case, check_append=False, launches=2)
     finally:
         lib.kpx_internal_set_decode_small(12, 12, 4)
+        lib.kpx_internal_set_decode_cluster(24)
+        lib.kpx_internal_set_decode_small_items(4)

@@ -114,9 +114,10 @@ def test_small_weights_keep_their_precision(native_libs):
         assert err <= bound, f"{dtype}: {err:.2e} > {bound:.2e}"
 
 
-@pytest.mark.parametrize("heads", [(4, 4), (4, 2), (8, 2), (7, 1), (8, 1)])
+@pytest.mark.parametrize("heads", [(4, 4), (4, 2), (6, 2), (8, 2), (7, 1), (8, 1)])
 def test_types_share_one_workspace(native_libs, heads):
-    """Long sequences (two levels of assembly) in f16, f32 and bf16 in turn on one workspace."""
+    """Long sequences (two levels of assembly) in f16, f32 and bf16 in turn on one workspace, in the line
+    of blocks: every launch leaves its pieces in the workspace's slots."""
     import torch
     from orinmllm_b200 import capi
     h, kv = heads
@@ -127,12 +128,20 @@ def test_types_share_one_workspace(native_libs, heads):
     capi.workspace_init(ws, nbytes)
     k, v = (torch.randn(n, kv * 128, generator=gen, device="cuda") for _ in range(2))
     q = torch.randn(1, h * 128, generator=gen, device="cuda")
-    for dtype in ("f16", "f32", "bf16", "f32", "f16"):
-        dt = kvtest.torch_dtype(dtype)
-        kd, vd, qd = (x.to(dt) for x in (k, v, q))
-        out = torch.full_like(qd, float("nan"))
-        lay = capi.layout_contiguous(capi.dtype_code(dt), kv, 128, 16, n // 16)
-        capi.paged_decode(out, qd, kd, vd, lay, None, 0, None, n, 1, h, 1 / math.sqrt(128), ws, nbytes)
-        assert capi.workspace_status(ws) == 0
-        ref = _reference(qd.view(h, 128), kd.view(n, kv, 128), vd.view(n, kv, 128))
-        _check(out.view(h, 128), ref, dtype, f"shared workspace {dtype}")
+    lib = capi.lib()
+    lib.kpx_internal_set_decode_cluster(0)
+    try:
+        for dtype in ("f16", "f32", "bf16", "f32", "f16"):
+            dt = kvtest.torch_dtype(dtype)
+            kd, vd, qd = (x.to(dt) for x in (k, v, q))
+            out = torch.full_like(qd, float("nan"))
+            before = ws.clone()
+            lay = capi.layout_contiguous(capi.dtype_code(dt), kv, 128, 16, n // 16)
+            capi.paged_decode(out, qd, kd, vd, lay, None, 0, None, n, 1, h, 1 / math.sqrt(128), ws, nbytes)
+            assert capi.workspace_status(ws) == 0
+            # (a piece of one head is half a KB; several hundred warps left one)
+            assert (ws != before).sum().item() > 100 * 512, "the launch did not use the workspace"
+            ref = _reference(qd.view(h, 128), kd.view(n, kv, 128), vd.view(n, kv, 128))
+            _check(out.view(h, 128), ref, dtype, f"shared workspace {dtype}")
+    finally:
+        lib.kpx_internal_set_decode_cluster(24)

@@ -66,6 +66,58 @@ def test_decode_wait_runs_out_and_the_workspace_recovers(native_libs, oracle, fo
     assert torch.equal(again.view(torch.uint8), good.view(torch.uint8)), "the launch after recovery differs"
 
 
+@pytest.mark.parametrize("dtype,heads,batch,length", [("f16", (32, 8), 1, 2000), ("bf16", (28, 4), 2, 500), ("f32", (12, 2), 1, 2000),
+                                                     ("f16", (32, 8), 18, 200)])
+@pytest.mark.parametrize("fused", [False, True])
+def test_cluster_form_wait_runs_out(native_libs, dtype, heads, batch, length, fused):
+    """A small launch (one cluster of CTAs per item): the warp that gives up still meets its CTA and its
+    cluster at every barrier, the rows of its item and no others come out as NaN, the status says
+    what happened, and the next launch is right."""
+    import torch
+    from orinmllm_b200 import capi
+    h, kv = heads
+    dt = kvtest.torch_dtype(dtype)
+    gen = torch.Generator(device="cuda").manual_seed(length)
+    width = length // 16 + 1
+    table = torch.randperm(batch * width, generator=gen, device="cuda").to(torch.int32).view(batch, width)
+    kp, vp = (torch.randn(batch * width, kv, 16, 128, generator=gen, device="cuda").to(dt) for _ in range(2))
+    q, k, v = (torch.randn(batch, n * 128, generator=gen, device="cuda").to(dt) for n in (h, kv, kv))
+    lens = torch.full((batch,), length, dtype=torch.int32, device="cuda")
+    sin, cos = (torch.empty((length + 1) * 128, device="cuda") for _ in range(2))
+    capi.sin_cos_cache(sin, cos, 128, length + 1, 1e6)
+    lay = capi.layout_paged(capi.dtype_code(dt), kv, 128, 16, batch * width)
+    nbytes = capi.decode_workspace_bytes(batch, h, kv)
+    ws = torch.empty(nbytes, dtype=torch.uint8, device="cuda")
+    capi.workspace_init(ws, nbytes)
+
+    def launch():
+        out = torch.full_like(q, 7.0)
+        if fused:
+            capi.rope_append_decode(out, q, k, v, sin, cos, kp, vp, lay, table, width, lens, batch, h, 1 / np.sqrt(128), ws, nbytes)
+        else:
+            capi.paged_decode(out, q, kp, vp, lay, table, width, lens, 0, batch, h, 1 / np.sqrt(128), ws, nbytes)
+        torch.cuda.synchronize()
+        return out.view(batch, h, 128)
+
+    good = launch()
+    assert capi.workspace_status(ws) == 0 and torch.isfinite(good.float()).all()
+    lib = capi.lib()
+    lib.kpx_internal_set_decode_fault(3000, 1)  # the second warp of the first item's first CTA
+    try:
+        broken = launch()
+    finally:
+        lib.kpx_internal_set_decode_fault(0, -1)
+    per_item = min(h // kv, 4 if dtype == "f32" else 8)  # query heads of an item
+    assert torch.isnan(broken[0, :per_item].float()).all()
+    rest = torch.ones(batch, h, dtype=torch.bool, device="cuda")
+    rest[0, :per_item] = False
+    assert torch.equal(broken[rest], good[rest])
+    assert capi.workspace_status(ws) == capi.KPX_ERR_DEVICE_TIMEOUT
+    again = launch()
+    assert capi.workspace_status(ws) == 0
+    assert torch.equal(again, good)
+
+
 @pytest.mark.parametrize("tile", [0, 1, 2], ids=["first_k_tile", "first_v_tile", "second_k_tile"])
 def test_prefill_wait_runs_out_and_the_next_call_is_right(native_libs, oracle, tile):
     """The tensor-core prefill kernel: one CTA never gets one of its tiles (the first K tile: the
