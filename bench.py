@@ -695,7 +695,7 @@ def run_gpu(args):
     line = {
         "metric": METRIC, "value": round(value, 1), "unit": "GB/s", "n_gpus": world, "steps": K,
         "warmup": W, "ms_per_step": round(ms_resident / K, 4), "higher_is_better": True,
-        "scaling": "weak", "vs_baseline": None, "dtype": "f16 storage, f32 arithmetic", "data": "synthetic",
+        "scaling": "weak", "vs_baseline": None, "dtype": "f16 storage; f16 products (weights as two terms), f32 sums", "data": "synthetic",
         "config": {"workload": "paged GQA decode, Qwen3-8B attention shape (32 Q / 8 KV heads, d=128), "
                                "fp16 KV, block 16, bs=64 per GPU, ctx U[128,4096], pool x1.25, "
                                "seeded random block table; step = RoPE+append+attend over 36 layers",
@@ -746,9 +746,9 @@ def run_gpu(args):
 
 # dram bytes (read+write) / algorithmic bytes of one decode launch, from the ncu capture
 # summarised in profiles/ (same kernel, same shape, one layer)
-TRAFFIC_RATIO = 1.020
+TRAFFIC_RATIO = 1.016
 TRAFFIC_NOTE = ("ncu dram__bytes_read+write of one launch of the overlapped form at this shape / algorithmic "
-                "bytes = 534.90 MB / 524.59 MB = 1.020 (the one-CTA-per-SM form: 1.017)")
+                "bytes = 532.72 MB / 524.59 MB = 1.016 (the one-CTA-per-SM form: 1.016)")
 
 
 def main():

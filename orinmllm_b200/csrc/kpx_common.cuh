@@ -70,9 +70,9 @@ int decode_rows(void* out, const void* q, const void* k_pool, const void* v_pool
 // ---- device-side helpers -------------------------------------------------------------
 #ifdef __CUDACC__
 
-// The kernels of a step follow each other on one stream and most run for a few microseconds.  They
-// are launched so that a kernel's CTAs may become resident while its predecessor on the stream
-// finishes (programmatic stream serialization): what a launch costs before its first instruction
+// The kernels of a step follow each other on one stream and most run for a few microseconds.  RoPE,
+// append (narrow tokens), the step's plan, decode, prefill and its merge are launched so that a
+// kernel's CTAs may become resident while its predecessor on the stream finishes (programmatic stream serialization): what a launch costs before its first instruction
 // runs then lies under the predecessor's end.  Every thread of such a kernel calls grid_wait()
 // before its first access to global memory, which returns when everything earlier on the stream
 // has completed and is visible; then grid_release() lets the successor's CTAs come.  A kernel so

@@ -6,20 +6,21 @@
 // translation unit per element type (kpx_decode_f16.cu, _bf16.cu, _f32.cu), each of which defines
 // dispatch_decode<T> once, so that the three sets of kernels compile side by side.
 //
-// Work decomposition.  The cache of sequence b holds len_b tokens in blocks of 16.
+// Work decomposition (all types).  The cache of sequence b holds len_b tokens in blocks of 16.
 // An "item" is one (sequence, kv head, query-head group) triple; its work is the
 // sequence's blocks.  All blocks of all items are laid on one line (sequence-major)
 // and cut into W equal contiguous ranges, one per *warp* of a persistent grid (one
-// CTA per SM, 12 warps per CTA for 16-bit caches), so every warp streams the same
-// number of bytes whatever the spread of sequence lengths.  A warp that covers an
+// CTA per SM, of 6 warps for fp32 caches and 8 for 16-bit ones), so every warp streams the
+// same number of bytes whatever the spread of sequence lengths.  A warp that covers an
 // item completely writes its output directly; an item cut by a range boundary
 // leaves one partial (running max, sum, un-normalised accumulator) per warp in the
 // workspace, and the warp that delivers the item's last piece (an atomic counter per item,
 // nobody waits) assembles the output; an item cut into more than 16 pieces is assembled in
 // two levels, 16 warps' pieces at a time.  One launch.  A launch that the host can tell to
-// be small (few blocks per warp) runs a second instantiation that cuts fewer, longer ranges.
+// be small (few blocks per warp) runs the cluster form (kpx_decode_cluster.cuh) or, where that is
+// not for it, cuts fewer, longer ranges (here: a second instantiation of the kernel).
 //
-// Each warp is its own producer and consumer: it owns two K and two V tile slots in
+// The kernel of fp32 caches.  Each warp is its own producer and consumer: it owns two K and two V tile slots in
 // shared memory, fetches the (block, kv head) tiles of its range through the block
 // table with cp.async.bulk (the TMA engine, completion on per-slot mbarriers), and
 // refills a slot the moment it has finished reading it -- the K slot right after

@@ -3,9 +3,9 @@
 // warp to arrive) with the two contractions on matrix instructions.
 //
 // Why matrix instructions: with up to eight query heads per KV head a 16-token tile (8 KB of K and
-// V) costs about 150 warp instructions here and cost 816 (four heads) to 1632 (five to eight heads,
-// in two passes over the tile) as packed fp32 FMAs, so that the instruction stream and not HBM set
-// the rate.  One warp owns a tile: S = Q K^T and O += P V are m16n8k16 products whose 16 rows are
+// V) costs about 350 warp instructions here, all of a launch counted (354, fp16), and cost 816 (four
+// heads) to 1632 (five to eight heads, in two passes over the tile) as packed fp32 FMAs, so that the
+// instruction stream and not HBM set the rate.  One warp owns a tile: S = Q K^T and O += P V are m16n8k16 products whose 16 rows are
 //   scores:  rows 0..7 = the eight query heads, rows 8..15 zero;
 //   output:  rows 0..7 = P_hi, rows 8..15 = P_lo of the same heads, p = P_hi + P_lo in two 16-bit
 //            terms, so that the second term costs no instruction of its own; the two row halves of
@@ -15,9 +15,10 @@
 //            times an infinity in V would be NaN).
 // Thread (g = lane / 4, t = lane % 4) holds head g and tokens 2t, 2t+1, 2t+8, 2t+9 of the scores:
 // the layout of the accumulator is that of the A operand of the second product, so weights never
-// leave their thread; the row maximum is two shuffles.  Q enters exactly as stored (bf16
-// rows times a power of two, Mma::row_scale); the softmax scale is applied to the fp32 scores.  The weights of fp16 caches are scaled by 2^12 (the
-// running sum with them), which keeps P_lo of small weights out of the subnormals.
+// leave their thread; the row maximum is two shuffles.  Q enters exactly as stored (bf16 rows times a
+// power of two, Mma::row_scale); the softmax scale is applied to the fp32 scores.  The weights of fp16
+// caches are scaled by 2^12 (the running sum with them), which keeps P_lo of small weights out of
+// the subnormals.
 //
 // Tiles arrive by TMA through 128-byte-swizzled tensor maps of the pools ([half row][16 tokens][64
 // elements], one 4 KB box), so that ldmatrix reads them without bank conflicts.  A strided cache
@@ -25,14 +26,14 @@
 // Eight warps per SM.  A launch that has the GPU to itself gives a warp one K and one V slot: 64 KB
 // in flight per SM keep HBM busy, and more only lengthens the queues, in which the SMs farther from
 // the memory they read fall behind until the last warp ends 25 us after the median one.  us per
-// launch with 1 / 2 / 3 slots: 32/8 heads, 64 sequences of 128..4096 tokens 100 / 104 / 110; 16 of
+// launch with 1 / 2 / 3 slots (alone): 32/8 heads, 64 sequences of 128..4096 tokens 100 / 104 / 110; 16 of
 // 8k..32k 215 / 226 / 237; one of 131072 107 / 110 / 113; 28/4 heads bf16, 64 sequences
 // 61 / 65 / 66.6.  (Twelve warps of two slots: 134; four warps of six: 126.)
 //
-// Measured, one layer of 64 sequences of 128..4096 tokens, before (packed FMAs) -> now: 28/4 heads
-// bf16 106 -> 61 us (277 MB; 4.5 TB/s), 32/8 heads fp16 105 -> 100 us (554 MB; 5.5 TB/s, bound by HBM
-// and the launch's ends); 256 sequences that share 1024 of 1344 tokens, 32/8: 228 -> 159 us.  Errors
-// against 64 bits are those of the output's rounding, as before (fp16 2.1e-4, bf16 1.7e-3).
+// Measured, us per launch in a graph, packed FMAs -> now: 64 sequences of 128..4096 tokens, 28/4 heads
+// bf16 93 -> 57 (the third term costs 1 of them), 32/8 fp16 100 -> 94, 32/8 bf16 101 -> 97 (third
+// term 3); 16 of 8k..32k, 32/8 fp16 213 -> 201; one of 131072 107 -> 95.  Errors against 64 bits are those
+// of the FMAs to five digits (rounding of the output included: fp16 2.1e-4, bf16 1.7e-3).
 #pragma once
 #include "kpx_decode_impl.cuh"
 #include "kpx_tma.cuh"
