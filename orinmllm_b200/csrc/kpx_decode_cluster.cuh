@@ -80,17 +80,23 @@ struct FmaTile {
       for (int i = 0; i < 8; ++i) acc[j][i] = make_float2(0.f, 0.f);
     }
   }
-  // rows of the group's heads, `stride` bytes apart; heads from `heads` on are zero
-  __device__ __forceinline__ void load_q(const uint8_t* rows, int stride, int heads, float qscale) {
+  // rows of the group's heads, `stride` bytes apart; heads from `heads` on are zero (loads only, as MmaTile)
+  __device__ __forceinline__ void load_q(const uint8_t* rows, int stride, int heads) {
 #pragma unroll
     for (int j = 0; j < QH; ++j)
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (j < heads) v = *reinterpret_cast<const float4*>(rows + int64_t(j) * stride + (c * 32 + sub * 4) * 4);
-        q[j][2 * c] = make_float2(v.x * qscale, v.y * qscale);
-        q[j][2 * c + 1] = make_float2(v.z * qscale, v.w * qscale);
+        q[j][2 * c] = make_float2(v.x, v.y);
+        q[j][2 * c + 1] = make_float2(v.z, v.w);
       }
+  }
+  __device__ __forceinline__ void scale_q(float qscale) {
+#pragma unroll
+    for (int j = 0; j < QH; ++j)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) q[j][i] = make_float2(q[j][i].x * qscale, q[j][i].y * qscale);
   }
   static __device__ __forceinline__ void row16(const uint8_t* row, int sub, float2 (&f)[8]) {
 #pragma unroll
@@ -266,7 +272,7 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
                           (int64_t(b) * p.num_q_heads + int64_t(kvh) * p.kv_mul + hg * QH) * kRowB + after_wait;
   Tile tile;
   tile.init(lane);
-  if constexpr (!kFused) tile.load_q(q_rows, kRowB, heads, p.qscale);
+  if constexpr (!kFused) tile.load_q(q_rows, kRowB, heads);
 
   // ids of 32 blocks at a time, one per lane
   int ids = 0;
@@ -321,8 +327,11 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
           p.sin_cache + int64_t(len) * kD + after_wait, p.cos_cache + int64_t(len) * kD + after_wait,
           row ? row + len / kBS : nullptr, len / kBS, stage, lane);
       __syncwarp();
-      tile.load_q(stage, Tile::kRowStride, heads, p.qscale);
+      tile.load_q(stage, Tile::kRowStride, heads);
+      tile.scale_q(p.qscale);
     }
+  } else {
+    tile.scale_q(p.qscale);  // (the tiles have been requested)
   }
 
   bool ok = true;

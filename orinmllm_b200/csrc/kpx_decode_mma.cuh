@@ -119,7 +119,7 @@ struct MmaTile {
   // at a time over the banks
   static constexpr int kRowStride = kRowB + 16;
   static constexpr bool kTensorMaps = true;
-  float by;           // what a product with the query rows is multiplied by to be a score (set by load_q)
+  float by;           // what a product with the query rows is multiplied by to be a score (set by scale_q)
   uint32_t qa[8][2];  // A fragments: k step s holds d = 16s + 2t, +1 and 16s + 8 + 2t, +1 of head g
   float acc[16][4];   // d = 8 * tile + 2t, +1 of head g: [0..1] the P_hi part, [2..3] the P_lo part
   float m, l;         // of head g; l: of the thread's own tokens until finish()
@@ -147,8 +147,9 @@ struct MmaTile {
     v_off = uint32_t(((lm & 1) * 8 + lr) * 128 + (((lm >> 1) ^ lr) << 4));
     reset();
   }
-  // rows of the group's heads, `stride` bytes apart; heads from `heads` on are zero
-  __device__ __forceinline__ void load_q(const uint8_t* rows, int stride, int heads, float qscale) {
+  // rows of the group's heads, `stride` bytes apart; heads from `heads` on are zero.  Loads only: nothing
+  // waits for them before scale_q, so that the requests of the first tiles go out meanwhile.
+  __device__ __forceinline__ void load_q(const uint8_t* rows, int stride, int heads) {
     const bool valid = g < heads;
     const uint32_t* qh = reinterpret_cast<const uint32_t*>(rows + (valid ? g : 0) * stride) + t;
 #pragma unroll
@@ -156,6 +157,9 @@ struct MmaTile {
       qa[s][0] = valid ? qh[8 * s] : 0u;
       qa[s][1] = valid ? qh[8 * s + 4] : 0u;
     }
+  }
+  // after load_q: the softmax scale, shared out between the rows and the scores
+  __device__ __forceinline__ void scale_q(float qscale) {
     by = M::score_scale(qscale);
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
       const float rows_by = M::row_scale(qscale);
@@ -518,7 +522,7 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
   auto load_q = [&]() {
     const int h0 = (cur.sub - cur.kvh * p.head_groups) * kMmaHeads;
     tile.load_q(static_cast<const uint8_t*>(p.q) + (int64_t(cur.b) * p.num_q_heads + cur.kvh * p.kv_mul + h0) * kRowB, kRowB,
-                p.kv_mul - h0, p.qscale);
+                p.kv_mul - h0);
   };
   // The first item's rows are requested here, before the first block id and the first tiles, so
   // that their latency (DRAM if nothing brought them to L2) runs under those.
@@ -589,10 +593,11 @@ paged_decode_mma_kernel(const DecodeParams p, const __grid_constant__ CUtensorMa
           p.sin_cache + int64_t(cur.len) * kD, p.cos_cache + int64_t(cur.len) * kD,
           cur.row ? cur.row + cur.len / kBS : nullptr, cur.len / kBS, stage, lane);
       __syncwarp();
-      tile.load_q(stage, C::kRowStride, p.kv_mul - hg * kMmaHeads, p.qscale);
+      tile.load_q(stage, C::kRowStride, p.kv_mul - hg * kMmaHeads);
     } else if (!first) {
       load_q();
     }
+    tile.scale_q(p.qscale);
     tile.reset();
   };
 
