@@ -9,10 +9,16 @@
 // from its index, reads one length, and its warps take equal shares of the item's blocks; the
 // pieces meet in shared memory, first those of a CTA's warps, then those of the cluster's CTAs
 // through distributed shared memory.  No workspace slot, no counter, no global round trip.
-// Measured, us per launch in a graph, line of blocks -> cluster form: fp16 32/8 heads, one sequence
+// Measured when it was built, us per launch in a graph, line of blocks -> cluster form: fp16 32/8 heads, one sequence
 // of 512 tokens 20.1 -> 5.5, 2000: 23.0 -> 7.4, 16384: 33.2 -> 22.5, 24000: 38.7 -> 31.2 (23 blocks
 // a warp: where the two come together); 8 sequences of 1500: 23.6 -> 13.8; 64 of 200 tokens in CTAs
 // of two warps: 13.9; fp32 12/2, 512 tokens: 17.0 -> 6.6, 4096: 22.3 -> 11.4.
+//
+// Since then a warp asks for the ids of its blocks together with the length (its share is every so-manieth block,
+// known without it), and the CTAs send their pieces to the one that assembles a head instead of being asked for
+// them one after the other.  Steps of RoPE + append + this, us before -> after: fp32 12/2, 512 tokens, 28 layers
+// 276 -> 241; fp16 32/8, 2000 tokens, 36 layers in a graph 361 -> 329 (0.4 a layer of it in the append); fp16 12/2, 8
+// sequences, 28 fused launches 274 -> 225.
 //
 // The arithmetic of a 16-token tile is a Tile type: MmaTile (16-bit caches, matrix instructions) or
 // FmaTile (fp32 caches, packed FMAs).
@@ -33,29 +39,24 @@ __device__ __forceinline__ uint32_t cluster_size() {
   asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void cluster_sync_all() {
-  __syncwarp();
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 }
-// 16 / 4 bytes of the shared memory of CTA `rank` of the cluster, at the address `addr` has here
-__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
-  float4 v;
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// 16 / 8 bytes into the shared memory of CTA `rank` of the cluster, at the address `addr` has here
+__device__ __forceinline__ void st_cluster_f4(uint32_t addr, uint32_t rank, float4 v) {
   asm volatile(
-      "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %4, %5;\n\t"
-      "ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [a];\n\t}"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "r"(addr), "r"(rank)
+      "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\t"
+      "st.shared::cluster.v4.f32 [a], {%2,%3,%4,%5};\n\t}" ::"r"(addr),
+      "r"(rank), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
       : "memory");
-  return v;
 }
-__device__ __forceinline__ float ld_cluster_f1(uint32_t addr, uint32_t rank) {
-  float v;
+__device__ __forceinline__ void st_cluster_f2(uint32_t addr, uint32_t rank, float x, float y) {
   asm volatile(
-      "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %1, %2;\n\tld.shared::cluster.f32 %0, [a];\n\t}"
-      : "=f"(v)
-      : "r"(addr), "r"(rank)
+      "{\n\t.reg .b32 a;\n\tmapa.shared::cluster.u32 a, %0, %1;\n\t"
+      "st.shared::cluster.v2.f32 [a], {%2,%3};\n\t}" ::"r"(addr),
+      "r"(rank), "f"(x), "f"(y)
       : "memory");
-  return v;
 }
 
 // One warp's tile arithmetic for fp32 caches: eight lanes share a token row (16 dims each), four
@@ -210,17 +211,23 @@ struct FmaTile {
   }
 };
 
+constexpr int kMaxCluster = 16;  // (above 8 only where the device says that such clusters fit)
+
 template <typename Tile, int NW, int NS>
 struct ClusterCfg {
+  // the largest cluster of this form: CTAs of two warps are for launches of many items, and four of them share an SM
+  static constexpr int kCtas = NW == 2 ? 8 : kMaxCluster;
   static constexpr int kTileB = kBS * Tile::kRowB;
   static constexpr int kWarpRingB = 2 * NS * kTileB;  // K slots then V slots; later the warp's piece
   static constexpr int kPieceFloats = Tile::QH * kD + 2 * Tile::QH;
   static constexpr int kOffBars = NW * kWarpRingB;
-  static constexpr int kOffSum = kOffBars + (NW * 2 * NS * 8 + 15) / 16 * 16;  // the CTA's piece
+  // pieces of the heads that this CTA assembles, one from each CTA: 128 floats, maximum, sum
+  static constexpr int kGotFloats = kD + 4, kGot = Tile::QH > kCtas ? Tile::QH : kCtas;
+  static constexpr int kOffGot = kOffBars + (NW * 2 * NS * 8 + 15) / 16 * 16;
   // Fused step only: as in MmaCfg, for the one warp that adds the new token and, for the query
   // rows, for all.
   static constexpr int kStageB = (Tile::QH + 2) * Tile::kRowStride + 16;
-  static constexpr int kOffStage = kOffSum + (kPieceFloats * 4 + 15) / 16 * 16;
+  static constexpr int kOffStage = kOffGot + kGot * kGotFloats * 4;
   static constexpr int kSmem = 1024 /*align slack*/ + kOffStage;
   static constexpr int kSmemFused = kSmem + NW * kStageB;
   static_assert(kWarpRingB % 1024 == 0 && kWarpRingB >= kPieceFloats * 4, "slots are aligned, and hold a piece");
@@ -250,48 +257,51 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
     }
   }
   __syncwarp();
+  if (ctas > 1) cluster_arrive();  // (waited for before this CTA writes to another's shared memory)
   const int64_t after_wait = grid_wait();
   grid_release();
 
-  // the item, and this warp's share of its blocks
+  // the item, and this warp's share of its blocks: every workers-th one, so that the ids of the first 32 can be
+  // asked for together with the length (a table row is there up to its width, whatever the length)
   const int item = int(blockIdx.x) / ctas;
   const int per_seq = p.num_kv_heads * p.head_groups;
   const int b = item / per_seq, sub_item = item - b * per_seq;
   const int kvh = sub_item / p.head_groups, hg = sub_item - kvh * p.head_groups;
   const int heads = min(QH, p.kv_mul - hg * QH);
+  const int workers = ctas * NW, worker = rank * NW + warp;
+  const int32_t* row =
+      p.block_table ? p.block_table + int64_t(p.row_index ? p.row_index[b] : b) * p.max_blocks_per_seq + after_wait : nullptr;
+  auto id_at = [&](int i) {  // of the i-th block of the share, 0 beyond the table's width
+    const int64_t at = worker + int64_t(i) * workers;
+    return row ? (at < p.max_blocks_per_seq ? __ldg(row + at) : 0) : int(at);
+  };
+  int ids = id_at(lane);  // 32 at a time, one per lane
+  const int len = seq_len_of(p, b);
   if (p.block_table && p.seq_lens && item % per_seq == 0 && rank == 0 && tid == 0 &&
       p.seq_lens[b] + p.len_bias > p.max_cached_tokens)
     atomicMax(p.status, KPX_ERR_INVALID_ARGUMENT);
-  const int len = seq_len_of(p, b);
   const int nblk = blocks_of(len);
-  const int workers = ctas * NW, worker = rank * NW + warp;
-  const int u0 = int(int64_t(nblk) * worker / workers), n = int(int64_t(nblk) * (worker + 1) / workers) - u0;
-  const int32_t* row =
-      p.block_table ? p.block_table + int64_t(p.row_index ? p.row_index[b] : b) * p.max_blocks_per_seq + after_wait : nullptr;
+  const int n = worker < nblk ? (nblk - worker + workers - 1) / workers : 0;
   const uint8_t* q_rows = static_cast<const uint8_t*>(p.q) +
                           (int64_t(b) * p.num_q_heads + int64_t(kvh) * p.kv_mul + hg * QH) * kRowB + after_wait;
   Tile tile;
   tile.init(lane);
   if constexpr (!kFused) tile.load_q(q_rows, kRowB, heads);
 
-  // ids of 32 blocks at a time, one per lane
-  int ids = 0;
-  auto load_ids = [&](int first) {
-    const int i = first + lane;
-    ids = 0;
-    if (i < n) {
-      ids = row ? __ldg(row + u0 + i) : u0 + i;
-      if (ids < 0 || (p.num_blocks > 0 && ids >= p.num_blocks)) {
-        atomicMax(p.status, KPX_ERR_INVALID_ARGUMENT);
-        ids = 0;
-      }
+  auto check_ids = [&](int first) {
+    if (first > 0) ids = id_at(first + lane);
+    if (first + lane >= n) {
+      ids = 0;
+    } else if (ids < 0 || (p.num_blocks > 0 && ids >= p.num_blocks)) {
+      atomicMax(p.status, KPX_ERR_INVALID_ARGUMENT);
+      ids = 0;
     }
     __syncwarp();
   };
   auto issue = [&](int i, bool withhold = false) {  // K and V tiles of block i of the share
-    if ((i & 31) == 0) load_ids(i);
+    if ((i & 31) == 0) check_ids(i);
     const int id = __shfl_sync(0xffffffffu, ids, i & 31);
-    const int rows = min(kBS, len - (u0 + i) * kBS);
+    const int rows = min(kBS, len - (worker + i * workers) * kBS);
 #pragma unroll
     for (int kv = 0; kv < 2; ++kv) {
       uint64_t* bar = bars + kv * NS + i % NS;
@@ -346,7 +356,7 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
   };
   for (int i = 0; i < n && ok; ++i) {
     const uint32_t phase = uint32_t(i / NS) & 1u;
-    const int rows = min(kBS, len - (u0 + i) * kBS);
+    const int rows = min(kBS, len - (worker + i * workers) * kBS);
     const bool linear = rows < kBS && !p.tile_contig;
     ok = wait_tile(bars + i % NS, phase);
     if (!ok) break;
@@ -389,61 +399,72 @@ decode_cluster_kernel(const DecodeParams p, const __grid_constant__ CUtensorMap 
   __syncwarp();
   if (!ok && lane < QH) piece[QH * kD + QH + lane] = NAN;
   __syncthreads();
-  float* sum = reinterpret_cast<float*>(smem + C::kOffSum);
-  auto merged = [&](int count, auto m_of, auto l_of, auto o_of, float& M, float& L) {
-    M = -INFINITY;
-    for (int i = 0; i < count; ++i) M = fmaxf(M, m_of(i));
-    L = 0.f;
-    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int i = 0; i < count; ++i) {
-      const float li = l_of(i);
-      const float w = li == 0.f ? 0.f : fast_exp2(m_of(i) - M);
-      const float4 v = o_of(i);
-      L = fmaf(li, w, L);
-      o.x = fmaf(v.x, w, o.x);
-      o.y = fmaf(v.y, w, o.y);
-      o.z = fmaf(v.z, w, o.z);
-      o.w = fmaf(v.w, w, o.w);
-    }
-    return o;
-  };
+  float* got = reinterpret_cast<float*>(smem + C::kOffGot);
   auto write_out = [&](int head, float4 o, float L) {
     const float inv = L == 0.f ? 0.f : 1.f / L;
     T* orow = static_cast<T*>(p.out) + (int64_t(b) * p.num_q_heads + int64_t(kvh) * p.kv_mul + hg * QH + head) * kD;
     Tile::write4(orow, 4 * lane, make_float4(o.x * inv, o.y * inv, o.z * inv, o.w * inv));
   };
+  if (ctas > 1) cluster_wait();  // every CTA of the cluster runs
   for (int head = warp; head < heads; head += NW) {  // a warp per head, a lane four dims
     auto at = [&](int i) { return reinterpret_cast<const float*>(smem + i * C::kWarpRingB); };
-    float M, L;
-    const float4 o = merged(
-        NW, [&](int i) { return at(i)[QH * kD + head]; }, [&](int i) { return at(i)[QH * kD + QH + head]; },
-        [&](int i) { return *reinterpret_cast<const float4*>(at(i) + head * kD + 4 * lane); }, M, L);
+    float m[NW], l[NW], M = -INFINITY, L = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+      m[i] = at(i)[QH * kD + head];
+      l[i] = at(i)[QH * kD + QH + head];
+      M = fmaxf(M, m[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < NW; ++i) {
+      const float w = l[i] == 0.f ? 0.f : fast_exp2(m[i] - M);
+      const float4 v = *reinterpret_cast<const float4*>(at(i) + head * kD + 4 * lane);
+      L = fmaf(l[i], w, L);
+      o.x = fmaf(v.x, w, o.x);
+      o.y = fmaf(v.y, w, o.y);
+      o.z = fmaf(v.z, w, o.z);
+      o.w = fmaf(v.w, w, o.w);
+    }
     if (ctas == 1) {
       write_out(head, o, L);
     } else {
-      *reinterpret_cast<float4*>(sum + head * kD + 4 * lane) = o;
-      if (lane == 0) {
-        sum[QH * kD + head] = M;
-        sum[QH * kD + QH + head] = L;
-      }
+      // Head h is assembled by CTA h modulo the cluster's size.  The pieces are sent there: fetched instead, each
+      // would be a trip of its own to another SM (and a second barrier keep the CTAs until all had fetched).
+      const uint32_t dst = smem_u32(got + ((head / ctas) * ctas + rank) * C::kGotFloats);
+      st_cluster_f4(dst + 16 * lane, head % ctas, o);
+      if (lane == 0) st_cluster_f2(dst + kD * 4, head % ctas, M, L);
     }
   }
   if (ctas == 1) return;
-  cluster_sync_all();
-  for (int i = warp; i * ctas + rank < heads; i += NW) {  // the cluster's CTAs share the heads
-    const int head = i * ctas + rank;
-    const uint32_t s = smem_u32(sum);
-    float M, L;
-    const float4 o = merged(
-        ctas, [&](int i) { return ld_cluster_f1(s + (QH * kD + head) * 4, i); },
-        [&](int i) { return ld_cluster_f1(s + (QH * kD + QH + head) * 4, i); },
-        [&](int i) { return ld_cluster_f4(s + (head * kD + 4 * lane) * 4, i); }, M, L);
-    write_out(head, o, L);
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  for (int i = warp; i * ctas + rank < heads; i += NW) {
+    const float* pieces = got + i * ctas * C::kGotFloats;
+    const bool on = lane < ctas;
+    const float m = on ? pieces[lane * C::kGotFloats + kD] : -INFINITY, l = on ? pieces[lane * C::kGotFloats + kD + 1] : 0.f;
+    float M = m;
+#pragma unroll
+    for (int k = C::kCtas / 2; k > 0; k >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, k));
+    M = __shfl_sync(0xffffffffu, M, 0);
+    const float mine = l == 0.f ? 0.f : fast_exp2(m - M);
+    float L = 0.f;
+    float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < C::kCtas; ++k) {
+      if (k >= ctas) break;
+      const float w = __shfl_sync(0xffffffffu, mine, k);
+      const float4 v = *reinterpret_cast<const float4*>(pieces + k * C::kGotFloats + 4 * lane);
+      L = fmaf(__shfl_sync(0xffffffffu, l, k), w, L);
+      o.x = fmaf(v.x, w, o.x);
+      o.y = fmaf(v.y, w, o.y);
+      o.z = fmaf(v.z, w, o.z);
+      o.w = fmaf(v.w, w, o.w);
+    }
+    write_out(i * ctas + rank, o, L);
   }
-  cluster_sync_all();  // nobody leaves while its shared memory is read
 }
-
-constexpr int kMaxCluster = 16;  // (above 8 only where the device says that such clusters fit)
 
 // A kernel form, made ready on the current device: its shared-memory size and cluster size allowed,
 // and how many clusters of 1, 2, 4, 8 and 16 CTAs the device holds at a time.
@@ -493,12 +514,12 @@ const ClusterForm* cluster_form() {
 // CTAs per item of a small launch in this form, 0 if it is not for it: all clusters run side by
 // side, and a warp's share stays within max_share blocks; beyond that the balance of the line
 // of blocks over all SMs is worth more than the short chain.
-inline int cluster_ctas(const DecodeParams& p, const ClusterForm& f, int warps, int max_share) {
+inline int cluster_ctas(const DecodeParams& p, const ClusterForm& f, int warps, int max_ctas, int max_share) {
   const int64_t items = int64_t(p.batch) * p.num_kv_heads * p.head_groups;
   const int64_t blocks = seq_blocks_bound(p);
   if (blocks < 0 || items > f.fit[0]) return 0;
   int lg = 0;
-  while (lg < 4 && items <= f.fit[lg + 1] && blocks > (int64_t(warps) << lg)) ++lg;  // no more warps than blocks
+  while ((1 << lg) < max_ctas && items <= f.fit[lg + 1] && blocks > (int64_t(warps) << lg)) ++lg;  // no more warps than blocks
   return blocks <= (int64_t(warps) << lg) * max_share ? 1 << lg : 0;
 }
 
@@ -507,7 +528,7 @@ template <typename Tile, int NW, int NS, bool kFused>
 int try_cluster_form(const DecodeParams& p, int max_share, cudaStream_t stream) {
   using C = ClusterCfg<Tile, NW, NS>;
   const ClusterForm* form = cluster_form<Tile, NW, NS, kFused>();
-  const int ctas = form ? cluster_ctas(p, *form, NW, max_share) : 0;
+  const int ctas = form ? cluster_ctas(p, *form, NW, C::kCtas, max_share) : 0;
   if (ctas == 0) return KPX_ERR_UNIMPLEMENTED;
   CUtensorMap map_k{}, map_v{};
   if (Tile::kTensorMaps) {
