@@ -2,6 +2,8 @@
 // block copy and block refcount updates.  All of these are pure data movement
 // (or element-wise fp32 math) bound by HBM bandwidth: 128-bit accesses,
 // grid-stride loops sized from the SM count.
+#include <type_traits>
+
 #include "kpx_common.cuh"
 
 namespace kpx {
@@ -24,13 +26,6 @@ inline LayoutDev to_dev(const kpx_kv_layout* l) {
   return d;
 }
 
-// Byte offset of element 0 of (slot, head) in a pool.
-__device__ __forceinline__ int64_t slot_head_offset_bytes(const LayoutDev& L, int64_t slot, int h) {
-  int64_t blk = slot / L.block_size;
-  int64_t off = slot - blk * L.block_size;
-  return (blk * L.block_stride + int64_t(h) * L.head_stride + off * L.token_stride) * L.elt_bytes;
-}
-
 // token index and remainder of work item i (32-bit division whenever the item count allows it)
 __device__ __forceinline__ void split_item(int64_t i, int per_tok, bool small, int64_t& t, int& r) {
   if (small) {
@@ -42,7 +37,8 @@ __device__ __forceinline__ void split_item(int64_t i, int per_tok, bool small, i
     r = int(i - t * per_tok);
   }
 }
-__device__ __forceinline__ int64_t slot_head_offset_bytes_fast(const LayoutDev& L, int64_t slot, int h) {
+// Byte offset of element 0 of (slot, head) in a pool.
+__device__ __forceinline__ int64_t slot_head_offset_bytes(const LayoutDev& L, int64_t slot, int h) {
   int64_t blk, off;
   if (uint64_t(slot) < 0x80000000ull) {
     const uint32_t b = uint32_t(slot) / uint32_t(L.block_size);
@@ -93,7 +89,7 @@ append_kernel(uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
       val[u] = __ldg(reinterpret_cast<const uint4*>((which ? v_src : k_src) + (t * vec_per_tok + vec) * 16));
       const int64_t slot = slot_mapping ? slot_mapping[t] : base_slot + t;
       if (slot < 0) continue;
-      dst[u] = (which ? v_pool : k_pool) + slot_head_offset_bytes_fast(L, slot, h) + vi * 16;
+      dst[u] = (which ? v_pool : k_pool) + slot_head_offset_bytes(L, slot, h) + vi * 16;
     }
 #pragma unroll
     for (int u = 0; u < kAppendUnroll; ++u)
@@ -104,8 +100,25 @@ append_kernel(uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
 // RoPE in place on Q and K rows, then optional append of the rotated K and of V.
 // One thread owns one rotation pair-group: 8 (16-bit) or 4 (fp32) consecutive j
 // of one head of one token, i.e. one 16-byte vector at j and one at j+head_size/2.
-template <typename T>
-__global__ void rope_append_kernel(T* __restrict__ q, T* __restrict__ k, const T* __restrict__ v,
+// Bound by the chain position -> sin / cos -> store up to about a hundred tokens, by how many such chains an SM
+// holds beyond.  kVec: sin, cos and norm weights lie on 16-byte boundaries and are fetched four floats at a time,
+// all before the norm, which takes their trip off the chain and costs registers (80 instead of 48).
+// Measured and dropped: two or four heads of a token per thread (fewer chains held: norm, 2048 tokens 15.3 / 18.7
+// against 14.8 us), kVec in 64 or 48 registers (spills: 19.1 / 24.7).
+template <int kN>
+__device__ __forceinline__ void load4(const float* p, float (&f)[kN]) {
+#pragma unroll
+  for (int i = 0; i < kN / 4; ++i) {
+    const float4 v = __ldg(reinterpret_cast<const float4*>(p) + i);
+    f[4 * i] = v.x;
+    f[4 * i + 1] = v.y;
+    f[4 * i + 2] = v.z;
+    f[4 * i + 3] = v.w;
+  }
+}
+template <typename T, bool kVec>
+__global__ void __launch_bounds__(256)
+rope_append_kernel(T* __restrict__ q, T* __restrict__ k, const T* __restrict__ v,
                                    int32_t q_heads, const int32_t* __restrict__ positions,
                                    int32_t pos_base, const float* __restrict__ sin_cache,
                                    const float* __restrict__ cos_cache, uint8_t* __restrict__ k_pool,
@@ -113,6 +126,17 @@ __global__ void rope_append_kernel(T* __restrict__ q, T* __restrict__ k, const T
                                    const int64_t* __restrict__ slot_mapping, int32_t num_tokens,
                                    LayoutDev L, const float* __restrict__ q_norm_w,
                                    const float* __restrict__ k_norm_w, float norm_eps) {
+  constexpr int E = Elt<T>::kPer16B;
+  const int hs = L.head_size;
+  const int groups_per_head = hs / 2 / E;  // pair-groups per head
+  const int kvh = L.num_kv_heads;
+  const int heads_q = q ? q_heads : 0;
+  const int heads_qk = heads_q + (k ? kvh : 0);
+  const int rot_per_tok = heads_qk * groups_per_head;
+  const int vvec_per_tok = (v && v_pool) ? kvh * hs / E : 0;
+  const int work_per_tok = rot_per_tok + vvec_per_tok;
+  const int64_t total = int64_t(num_tokens) * work_per_tok;
+  const bool small = total < (int64_t(1) << 31);
   const int64_t after_wait = grid_wait();
   grid_release();
   q += q ? after_wait : 0;
@@ -124,41 +148,45 @@ __global__ void rope_append_kernel(T* __restrict__ q, T* __restrict__ k, const T
   cos_cache += after_wait;
   q_norm_w += q_norm_w ? after_wait : 0;
   k_norm_w += k_norm_w ? after_wait : 0;
-  constexpr int E = Elt<T>::kPer16B;
-  const int hs = L.head_size;
-  const int groups_per_head = hs / 2 / E;  // pair-groups per head
-  const int kvh = L.num_kv_heads;
-  const int heads_qk = (q ? q_heads : 0) + (k ? kvh : 0);
-  const int vvec_per_tok = (v && v_pool) ? kvh * hs / E : 0;
-  const int work_per_tok = heads_qk * groups_per_head + vvec_per_tok;
-  const int64_t total = int64_t(num_tokens) * work_per_tok;
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < total;
        i += int64_t(gridDim.x) * blockDim.x) {
-    int64_t t = i / work_per_tok;
-    int r = int(i - t * work_per_tok);
-    int64_t slot = slot_mapping ? slot_mapping[t] : -1;
-    if (r >= heads_qk * groups_per_head) {
+    int64_t t;
+    int r;
+    split_item(i, work_per_tok, small, t, r);
+    const int64_t slot = slot_mapping ? slot_mapping[t] : -1;
+    if (r >= rot_per_tok) {
       // plain V copy into the pool
+      const int vec = r - rot_per_tok;
+      const int h = vec / (hs / E);
+      const int vi = vec - h * (hs / E);
+      const uint4 row = __ldg(reinterpret_cast<const uint4*>(v + (t * kvh + h) * int64_t(hs)) + vi);
       if (slot < 0) continue;
-      int vec = r - heads_qk * groups_per_head;
-      int h = vec / (hs / E);
-      int vi = vec - h * (hs / E);
-      const uint4* src = reinterpret_cast<const uint4*>(v + (t * kvh + h) * int64_t(hs)) + vi;
-      *reinterpret_cast<uint4*>(v_pool + slot_head_offset_bytes(L, slot, h) + vi * 16) = __ldg(src);
+      *reinterpret_cast<uint4*>(v_pool + slot_head_offset_bytes(L, slot, h) + vi * 16) = row;
       continue;
     }
-    int head = r / groups_per_head;
-    int g = r - head * groups_per_head;
-    bool is_k = q ? head >= q_heads : true;
-    int h = is_k ? head - (q ? q_heads : 0) : head;
-    T* row = is_k ? k + (t * kvh + h) * int64_t(hs) : q + (t * q_heads + h) * int64_t(hs);
+    const int head = r / groups_per_head;
+    const int g = r - head * groups_per_head;
+    const bool is_k = head >= heads_q;
+    T* row = is_k ? k + (t * kvh + (head - heads_q)) * int64_t(hs) : q + (t * q_heads + head) * int64_t(hs);
     const int32_t pos = (positions ? positions[t] : int32_t(t)) + pos_base;
-    uint4 lo_raw = *reinterpret_cast<const uint4*>(row + g * E);
-    uint4 hi_raw = *reinterpret_cast<const uint4*>(row + hs / 2 + g * E);
+    const uint4 lo_raw = *reinterpret_cast<const uint4*>(row + g * E);
+    const uint4 hi_raw = *reinterpret_cast<const uint4*>(row + hs / 2 + g * E);
+    // of pair j the tables hold elements 2 j (used) and 2 j + 1
+    const float* sin_row = sin_cache + int64_t(pos) * hs + 2 * g * E;
+    const float* cos_row = cos_cache + int64_t(pos) * hs + 2 * g * E;
+    const float* norm_w = is_k ? k_norm_w : q_norm_w;
+    float sn[2 * E], cs[2 * E], wl[E], wh[E];
+    if constexpr (kVec) {
+      load4(sin_row, sn);
+      load4(cos_row, cs);
+      if (norm_w) {
+        load4(norm_w + g * E, wl);
+        load4(norm_w + hs / 2 + g * E, wh);
+      }
+    }
     float lo[E], hi[E];
     Elt<T>::unpack(lo_raw, lo);
     Elt<T>::unpack(hi_raw, hi);
-    const float* norm_w = is_k ? k_norm_w : q_norm_w;
     if (norm_w) {
       // per-head RMSNorm before the rotation (Qwen3 q/k norm): the head's groups_per_head
       // threads are consecutive lanes of one warp and walk this path together
@@ -172,30 +200,29 @@ __global__ void rope_append_kernel(T* __restrict__ q, T* __restrict__ k, const T
       const float rs = 1.f / sqrtf(ss / float(hs) + norm_eps);
 #pragma unroll
       for (int e = 0; e < E; ++e) {
-        lo[e] = __ldg(norm_w + g * E + e) * (rs * lo[e]);
-        hi[e] = __ldg(norm_w + hs / 2 + g * E + e) * (rs * hi[e]);
+        lo[e] = (kVec ? wl[e] : __ldg(norm_w + g * E + e)) * (rs * lo[e]);
+        hi[e] = (kVec ? wh[e] : __ldg(norm_w + hs / 2 + g * E + e)) * (rs * hi[e]);
       }
     }
     __align__(16) T lo_out[E];
     __align__(16) T hi_out[E];
 #pragma unroll
     for (int e = 0; e < E; ++e) {
-      int j = g * E + e;
-      float fci = __ldg(sin_cache + int64_t(pos) * hs + 2 * j);
-      float fcr = __ldg(cos_cache + int64_t(pos) * hs + 2 * j);
+      const float fci = kVec ? sn[2 * e] : __ldg(sin_row + 2 * e);
+      const float fcr = kVec ? cs[2 * e] : __ldg(cos_row + 2 * e);
       // v0*cos - v1*sin and v0*sin + v1*cos with separately rounded products, as
       // the reference CPU statement computes them (no FMA contraction).
-      float r0 = __fsub_rn(__fmul_rn(lo[e], fcr), __fmul_rn(hi[e], fci));
-      float r1 = __fadd_rn(__fmul_rn(lo[e], fci), __fmul_rn(hi[e], fcr));
+      const float r0 = __fsub_rn(__fmul_rn(lo[e], fcr), __fmul_rn(hi[e], fci));
+      const float r1 = __fadd_rn(__fmul_rn(lo[e], fci), __fmul_rn(hi[e], fcr));
       lo_out[e] = Elt<T>::from_float(r0);
       hi_out[e] = Elt<T>::from_float(r1);
     }
-    uint4 lo_w = *reinterpret_cast<uint4*>(lo_out);
-    uint4 hi_w = *reinterpret_cast<uint4*>(hi_out);
+    const uint4 lo_w = *reinterpret_cast<uint4*>(lo_out);
+    const uint4 hi_w = *reinterpret_cast<uint4*>(hi_out);
     *reinterpret_cast<uint4*>(row + g * E) = lo_w;
     *reinterpret_cast<uint4*>(row + hs / 2 + g * E) = hi_w;
     if (is_k && k_pool && slot >= 0) {
-      uint8_t* dst = k_pool + slot_head_offset_bytes(L, slot, h);
+      uint8_t* dst = k_pool + slot_head_offset_bytes(L, slot, head - heads_q);
       *reinterpret_cast<uint4*>(dst + g * 16) = lo_w;
       *reinterpret_cast<uint4*>(dst + (hs / 2) * sizeof(T) + g * 16) = hi_w;
     }
@@ -368,8 +395,8 @@ inline int grid_for(int64_t work_items, int threads) {
 // Grid of a grid-stride kernel capped at exactly what the SMs hold at once (from the occupancy
 // calculator, looked up once per kernel): a cap above that runs the surplus CTAs as a second,
 // partly filled wave.
-template <typename Kernel>
-inline int resident_grid_for(Kernel kernel, int64_t work_items, int threads) {
+template <auto kernel>
+inline int resident_grid_for(int64_t work_items, int threads) {
   static int per_sm = 0;
   if (per_sm == 0) {
     int n = 0;
@@ -431,6 +458,11 @@ extern "C" int kpx_append(void* k_pool, void* v_pool, const kpx_kv_layout* layou
   return cuda_status(cudaGetLastError());
 }
 
+// Up to this many threads the form that fetches tables and weights early is launched where there is a norm.
+// norm + RoPE + append, fp16 32/8 heads, us, that form / the other: 1 token 1.96 / 2.37, 64 2.35 / 2.65, 256
+// 4.00 / 4.52, 777 7.15 / 7.40, 2048 (0.9 million threads) 14.4 / 14.8, 16384 113 / 98.  Without a norm there is no
+// more to fetch than the chain brings anyway: bf16 28/4 1.89 / 1.81, 2.14 / 2.06, fp32 1.74 / 1.66, 1.99 / 1.93.
+constexpr int64_t kEarlyTables = 1000000;
 template <typename T>
 static int launch_rope(void* q, void* k, const void* v, int32_t q_heads, const int32_t* positions,
                        int32_t pos_base, const float* sin_cache, const float* cos_cache, void* k_pool, void* v_pool,
@@ -441,15 +473,23 @@ static int launch_rope(void* q, void* k, const void* v, int32_t q_heads, const i
   int groups = L.head_size / 2 / E;
   // the fused norm sums a head's squares across the `groups` consecutive lanes that hold it
   if ((q_norm_w || k_norm_w) && (groups > 32 || (groups & (groups - 1)))) return KPX_ERR_UNIMPLEMENTED;
-  int64_t work = int64_t(num_tokens) *
-                 (((q ? q_heads : 0) + (k ? L.num_kv_heads : 0)) * groups +
-                  ((v && v_pool) ? L.num_kv_heads * L.head_size / E : 0));
-  if (work == 0) return KPX_OK;
-  const int threads = 256;
-  return launch_chained(rope_append_kernel<T>, dim3(resident_grid_for(rope_append_kernel<T>, work, threads)), dim3(threads), 0,
-                        stream, static_cast<T*>(q), static_cast<T*>(k), static_cast<const T*>(v), q_heads, positions, pos_base,
-                        sin_cache, cos_cache, static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool), slot_mapping,
-                        num_tokens, L, q_norm_w, k_norm_w, norm_eps);
+  if (num_tokens == 0) return KPX_OK;
+  const int heads = (q ? q_heads : 0) + (k ? L.num_kv_heads : 0);
+  const int vvecs = (v && v_pool) ? L.num_kv_heads * L.head_size / E : 0;
+  if (heads * groups + vvecs == 0) return KPX_OK;
+  const int64_t work = int64_t(num_tokens) * (heads * groups + vvecs);
+  auto launch = [&](auto early) {
+    constexpr auto kernel = rope_append_kernel<T, decltype(early)::value>;
+    const int threads = 256;
+    return launch_chained(kernel, dim3(resident_grid_for<kernel>(work, threads)), dim3(threads), 0, stream, static_cast<T*>(q),
+                          static_cast<T*>(k), static_cast<const T*>(v), q_heads, positions, pos_base, sin_cache, cos_cache,
+                          static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool), slot_mapping, num_tokens, L, q_norm_w,
+                          k_norm_w, norm_eps);
+  };
+  const bool aligned = ((reinterpret_cast<uintptr_t>(sin_cache) | reinterpret_cast<uintptr_t>(cos_cache) |
+                         reinterpret_cast<uintptr_t>(q_norm_w) | reinterpret_cast<uintptr_t>(k_norm_w)) & 15) == 0;
+  if (aligned && (q_norm_w || k_norm_w) && work <= kEarlyTables) return launch(std::true_type());
+  return launch(std::false_type());
 }
 
 extern "C" int kpx_rope_append(void* q, void* k, const void* v, int32_t q_heads,
