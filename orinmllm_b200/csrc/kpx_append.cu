@@ -229,6 +229,138 @@ rope_append_kernel(T* __restrict__ q, T* __restrict__ k, const T* __restrict__ v
   }
 }
 
+// The same for many tokens, 16-bit rows of 128: a CTA takes kTokens tokens and brings what they share into
+// shared memory once, sin and cos of its tokens (their used halves) and the norm weights.  The flat form above is
+// bound by its L1 wavefronts there: every thread reads 128 bytes of tables, every other float unused, for 32 bytes
+// of rows, 64 of a warp's 96 wavefronts.
+// us, flat form -> this, norm fp16 32/8 heads: 777 tokens 7.1 -> 6.2, 2048 14.5 -> 10.4, 16384 97 -> 89; no norm
+// bf16 28/4: 5.05 -> 3.9, 9.7 -> 6.3, 68 -> 60.  (2048 tokens with 1 / 2 / 4 tokens a CTA: 11.5 / 10.4 / 14.6; 256
+// threads 14.3; one or four items in flight a thread 12.2 / 13.3.)
+constexpr int kRowsThreads = 128, kRowsBatch = 2;
+template <typename T, int kTokens>
+__global__ void __launch_bounds__(kRowsThreads)
+rope_rows_kernel(T* __restrict__ q, T* __restrict__ k, const T* __restrict__ v, int32_t q_heads,
+                 const int32_t* __restrict__ positions, int32_t pos_base, const float* __restrict__ sin_cache,
+                 const float* __restrict__ cos_cache, uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
+                 const int64_t* __restrict__ slot_mapping, int32_t num_tokens, LayoutDev L,
+                 const float* __restrict__ q_norm_w, const float* __restrict__ k_norm_w, float norm_eps) {
+  constexpr int hs = 128, E = 8, kGroups = hs / 2 / E;
+  static_assert(kTokens <= 2, "a token's number within the CTA is one comparison");
+  __shared__ __align__(16) float s_sin[kTokens][hs / 2], s_cos[kTokens][hs / 2], s_w[2][hs];
+  __shared__ int64_t s_slot[kTokens];
+  const int64_t after_wait = grid_wait();
+  grid_release();
+  q += q ? after_wait : 0;
+  k += k ? after_wait : 0;
+  v += v ? after_wait : 0;
+  positions += positions ? after_wait : 0;
+  slot_mapping += slot_mapping ? after_wait : 0;
+  sin_cache += after_wait;
+  cos_cache += after_wait;
+  q_norm_w += q_norm_w ? after_wait : 0;
+  k_norm_w += k_norm_w ? after_wait : 0;
+  const int tid = threadIdx.x;
+  const int64_t tok0 = int64_t(blockIdx.x) * kTokens;
+  const int tokens = int(min(int64_t(kTokens), num_tokens - tok0));
+  const int kvh = L.num_kv_heads;
+  const int heads_q = q ? q_heads : 0, heads_qk = heads_q + (k ? kvh : 0);
+  const int rot = heads_qk * kGroups, per_tok = rot + ((v && v_pool) ? kvh * hs / E : 0);
+  const int total = tokens * per_tok;
+  {
+#pragma unroll
+    for (int i = tid; i < kTokens * hs / 2; i += kRowsThreads) {
+      const int t = i / (hs / 2), c = i % (hs / 2);
+      if (t >= tokens) break;
+      const int64_t at = int64_t((positions ? positions[tok0 + t] : int32_t(tok0 + t)) + pos_base) * hs + 2 * c;
+      s_sin[t][c] = __ldg(sin_cache + at);
+      s_cos[t][c] = __ldg(cos_cache + at);
+    }
+    if (tid < tokens) s_slot[tid] = slot_mapping ? slot_mapping[tok0 + tid] : -1;
+#pragma unroll
+    for (int i = tid; i < 2 * hs; i += kRowsThreads) {
+      const float* w = i < hs ? q_norm_w : k_norm_w;
+      if (w) s_w[i / hs][i % hs] = __ldg(w + i % hs);
+    }
+  }
+  // Items of the CTA's tokens as the flat form numbers them.  The group of a head is the same for all items of a
+  // thread, and its lanes are consecutive lanes of one warp (all counts are multiples of kGroups).
+  const int g = tid % kGroups;
+  for (int i0 = tid; i0 - tid < total; i0 += kRowsThreads * kRowsBatch) {
+    uint4 lo_raw[kRowsBatch], hi_raw[kRowsBatch];
+    T* row[kRowsBatch];
+    int tok[kRowsBatch], head[kRowsBatch];  // head >= heads_qk: V, its vector is head * kGroups + g beyond the rotations
+#pragma unroll
+    for (int u = 0; u < kRowsBatch; ++u) {
+      const int i = i0 + u * kRowsThreads;
+      tok[u] = -1;
+      if (i >= total) continue;
+      const int t = kTokens == 2 && i >= per_tok ? 1 : 0;
+      const int r = i - t * per_tok;
+      tok[u] = t;
+      head[u] = r / kGroups;
+      const int64_t tt = tok0 + t;
+      if (r >= rot) {
+        lo_raw[u] = __ldg(reinterpret_cast<const uint4*>(v + tt * kvh * int64_t(hs)) + (r - rot));
+      } else {
+        row[u] = head[u] >= heads_q ? k + (tt * kvh + (head[u] - heads_q)) * int64_t(hs) : q + (tt * q_heads + head[u]) * int64_t(hs);
+        lo_raw[u] = *reinterpret_cast<const uint4*>(row[u] + g * E);
+        hi_raw[u] = *reinterpret_cast<const uint4*>(row[u] + hs / 2 + g * E);
+      }
+    }
+    if (i0 == tid) __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kRowsBatch; ++u) {
+      if (tok[u] < 0) continue;
+      const int64_t slot = s_slot[tok[u]];
+      if (head[u] >= heads_qk) {
+        const int vec = head[u] * kGroups + g - rot;
+        if (slot >= 0)
+          *reinterpret_cast<uint4*>(v_pool + slot_head_offset_bytes(L, slot, vec / (hs / E)) + vec % (hs / E) * 16) = lo_raw[u];
+        continue;
+      }
+      const bool is_k = head[u] >= heads_q;
+      float lo[E], hi[E];
+      Elt<T>::unpack(lo_raw[u], lo);
+      Elt<T>::unpack(hi_raw[u], hi);
+      if (is_k ? k_norm_w : q_norm_w) {
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) ss = fmaf(hi[e], hi[e], fmaf(lo[e], lo[e], ss));
+        const uint32_t head_mask = 0xffu << (tid & 24);
+#pragma unroll
+        for (int m = 1; m < kGroups; m <<= 1) ss += __shfl_xor_sync(head_mask, ss, m);
+        const float rs = 1.f / sqrtf(ss / float(hs) + norm_eps);
+        const float* w = s_w[is_k];
+#pragma unroll
+        for (int e = 0; e < E; ++e) {
+          lo[e] = w[g * E + e] * (rs * lo[e]);
+          hi[e] = w[hs / 2 + g * E + e] * (rs * hi[e]);
+        }
+      }
+      __align__(16) T lo_out[E];
+      __align__(16) T hi_out[E];
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        // products rounded separately, as above
+        const float fci = s_sin[tok[u]][g * E + e], fcr = s_cos[tok[u]][g * E + e];
+        const float r0 = __fsub_rn(__fmul_rn(lo[e], fcr), __fmul_rn(hi[e], fci));
+        const float r1 = __fadd_rn(__fmul_rn(lo[e], fci), __fmul_rn(hi[e], fcr));
+        lo_out[e] = Elt<T>::from_float(r0);
+        hi_out[e] = Elt<T>::from_float(r1);
+      }
+      const uint4 lo_w = *reinterpret_cast<uint4*>(lo_out);
+      const uint4 hi_w = *reinterpret_cast<uint4*>(hi_out);
+      *reinterpret_cast<uint4*>(row[u] + g * E) = lo_w;
+      *reinterpret_cast<uint4*>(row[u] + hs / 2 + g * E) = hi_w;
+      if (is_k && k_pool && slot >= 0) {
+        uint8_t* dst = k_pool + slot_head_offset_bytes(L, slot, head[u] - heads_q);
+        *reinterpret_cast<uint4*>(dst + g * 16) = lo_w;
+        *reinterpret_cast<uint4*>(dst + hs + g * 16) = hi_w;
+      }
+    }
+  }
+}
+
 // ---- token-walking form of the plain append ------------------------------------------
 // When a token's work items fit one CTA (<= 1024), thread r of the CTA does item r of every
 // token the CTA visits (tokens blockIdx.x, blockIdx.x + gridDim.x, ...).  A thread's role
@@ -463,6 +595,10 @@ extern "C" int kpx_append(void* k_pool, void* v_pool, const kpx_kv_layout* layou
 // 4.00 / 4.52, 777 7.15 / 7.40, 2048 (0.9 million threads) 14.4 / 14.8, 16384 113 / 98.  Without a norm there is no
 // more to fetch than the chain brings anyway: bf16 28/4 1.89 / 1.81, 2.14 / 2.06, fp32 1.74 / 1.66, 1.99 / 1.93.
 constexpr int64_t kEarlyTables = 1000000;
+// From kRowsFrom tokens on 16-bit rows of 128 take rope_rows_kernel (256 tokens: 4.4 / 2.8 us against 3.9 / 2.7 of the
+// flat forms; 512: 5.0 / 3.1 against 5.3 / 3.8), from kRowsPairs on with two tokens a CTA (777: 7.0 / 4.4 against 6.2 /
+// 3.9 with one; 2048: 10.4 / 6.3 against 11.5 / 7.3).
+constexpr int kRowsFrom = 400, kRowsPairs = 1400;
 template <typename T>
 static int launch_rope(void* q, void* k, const void* v, int32_t q_heads, const int32_t* positions,
                        int32_t pos_base, const float* sin_cache, const float* cos_cache, void* k_pool, void* v_pool,
@@ -486,6 +622,16 @@ static int launch_rope(void* q, void* k, const void* v, int32_t q_heads, const i
                           static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool), slot_mapping, num_tokens, L, q_norm_w,
                           k_norm_w, norm_eps);
   };
+  if constexpr (sizeof(T) == 2) {
+    auto launch_rows = [&](auto kernel, int tokens) {
+      return launch_chained(kernel, dim3(unsigned((int64_t(num_tokens) + tokens - 1) / tokens)), dim3(kRowsThreads), 0, stream,
+                            static_cast<T*>(q), static_cast<T*>(k), static_cast<const T*>(v), q_heads, positions, pos_base,
+                            sin_cache, cos_cache, static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool), slot_mapping,
+                            num_tokens, L, q_norm_w, k_norm_w, norm_eps);
+    };
+    if (L.head_size == 128 && num_tokens >= kRowsFrom)
+      return num_tokens < kRowsPairs ? launch_rows(rope_rows_kernel<T, 1>, 1) : launch_rows(rope_rows_kernel<T, 2>, 2);
+  }
   const bool aligned = ((reinterpret_cast<uintptr_t>(sin_cache) | reinterpret_cast<uintptr_t>(cos_cache) |
                          reinterpret_cast<uintptr_t>(q_norm_w) | reinterpret_cast<uintptr_t>(k_norm_w)) & 15) == 0;
   if (aligned && (q_norm_w || k_norm_w) && work <= kEarlyTables) return launch(std::true_type());
