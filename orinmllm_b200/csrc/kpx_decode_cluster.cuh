@@ -18,7 +18,7 @@
 // known without it), and the CTAs send their pieces to the one that assembles a head instead of being asked for
 // them one after the other.  Steps of RoPE + append + this, us before -> after: fp32 12/2, 512 tokens, 28 layers
 // 276 -> 241; fp16 32/8, 2000 tokens, 36 layers in a graph 361 -> 329 (0.4 a layer of it in the append); fp16 12/2, 8
-// sequences, 28 fused launches 274 -> 225.
+// sequences, 28 fused launches 274 -> 225 (214 with the new token's rows fetched together, stage_new_token).
 //
 // The arithmetic of a 16-token tile is a Tile type: MmaTile (16-bit caches, matrix instructions) or
 // FmaTile (fp32 caches, packed FMAs).
