@@ -1,9 +1,9 @@
 // Chunked-prefill attention on the 5th-generation tensor cores (tcgen05 + TMEM), 16-bit caches.
 //
 // An item is 128 query rows that share a KV head: 128 / n tokens times the n query heads of the head's
-// group (a group wider than 128 is cut into equal ones), so that a short tail of a prompt fills rows with heads instead of leaving a tile
-// per head nearly empty.  A unit of work is two neighbouring items of one sequence.  A cluster
-// of two CTAs (two SMs) works through the units the host dealt to it; CTA r holds the rows of item r
+// group (a group wider than 128 is cut into equal ones), so that a short tail of a prompt fills rows
+// with heads instead of leaving a tile per head nearly empty.  A unit of work is two neighbouring items
+// of one sequence.  A cluster of two CTAs (two SMs) works through the units the host dealt to it; CTA r holds the rows of item r
 // and half of every K / V tile, and one tcgen05.mma of the pair (cta_group::2, 256 rows) reads both
 // halves, so each K / V byte crosses L2 once for 256 rows.
 // What bounds it is the tensor pipe: 24 products of 128 x 128 x 16 per SM and 128-key tile (8 scores,
@@ -1142,9 +1142,24 @@ int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool,
       std::vector<Unit> parts;
       parts.reserve(units.size() + kMaxPartSlots);
       int slot = 0;
-      if (longest > even) {  // a few long units: none longer than an even share
-        const int cap = std::max(2, int(even));
-        for (const Unit& d : units) cut_unit(d, std::min(kMaxParts, (d.tile1 + cap - 1) / cap), slot, parts, merges);
+      if (longest > even) {
+        // A few long units: no part longer than a k-th of the longest, k by the rounds that the parts make.  (Cut to
+        // an even share instead, whatever the rounds: 512 tokens behind 3584, 32/8 heads, 64 units on 74 clusters, 51 us
+        // against 42; 256 behind 8192, 28/4, 71 against 59; 256 behind 3840, 32/8, 41 against 36.)
+        int cap = 0, best = load;
+        for (int k = 2; k <= kMaxParts; ++k) {
+          const int c = (longest + k - 1) / k;
+          int64_t count = 0;
+          for (const Unit& d : units) count += (d.tile1 + c - 1) / c;
+          const int64_t rounds = (count + clusters - 1) / clusters, mean = (tiles + count * kUnitCost + count - 1) / count;
+          const int cost = int(std::max<int64_t>(c + kUnitCost, rounds * mean)) + kMergeCost;
+          if (cost < best) {
+            best = cost;
+            cap = c;
+          }
+        }
+        if (cap > 0)
+          for (const Unit& d : units) cut_unit(d, std::min(kMaxParts, (d.tile1 + cap - 1) / cap), slot, parts, merges);
       } else {  // many units of like length and a thin last round: the shortest, a round's remainder, are cut
         const int rest = n % clusters;
         const std::vector<int32_t> by_length = longest_first(units);
