@@ -66,6 +66,7 @@ struct FmaTile {
   using T = float;
   static constexpr int QH = QH_, kRowB = kD * 4, kRowStride = kD * 4 + 16;
   static constexpr bool kTensorMaps = false;
+  static constexpr int kWidestForm = 6;  // warps of the cluster form that has an SM to itself
   static constexpr float kWeightBias = 0.f;
   float2 q[QH][8], acc[QH][8];
   float m[QH], l[QH];
@@ -215,8 +216,12 @@ constexpr int kMaxCluster = 16;  // (above 8 only where the device says that suc
 
 template <typename Tile, int NW, int NS>
 struct ClusterCfg {
-  // the largest cluster of this form: CTAs of two warps are for launches of many items, and four of them share an SM
-  static constexpr int kCtas = NW == 2 ? 8 : kMaxCluster;
+  // The largest cluster of this form.  The narrow forms are for launches of more items than SMs (a launch that wants
+  // sixteen CTAs an item has gone to the widest form before), and their CTAs share an SM: places for the pieces of
+  // sixteen CTAs took the fused form of four warps from two CTAs an SM to one (fp16 32/8 heads, 28 sequences of
+  // 100..500 tokens 13.5 -> 18.3 us), and that of three (fp32, 20 of 50..250: 14.2 -> 19.5).
+  static constexpr int kPerSm = Tile::kWidestForm / NW, kPerSmFused = NW == 2 ? 3 : kPerSm;
+  static constexpr int kCtas = kPerSm > 1 ? 8 : kMaxCluster;
   static constexpr int kTileB = kBS * Tile::kRowB;
   static constexpr int kWarpRingB = 2 * NS * kTileB;  // K slots then V slots; later the warp's piece
   static constexpr int kPieceFloats = Tile::QH * kD + 2 * Tile::QH;
@@ -231,6 +236,9 @@ struct ClusterCfg {
   static constexpr int kSmem = 1024 /*align slack*/ + kOffStage;
   static constexpr int kSmemFused = kSmem + NW * kStageB;
   static_assert(kWarpRingB % 1024 == 0 && kWarpRingB >= kPieceFloats * 4, "slots are aligned, and hold a piece");
+  static constexpr int kSmB = 228 * 1024, kReservedB = 1024;  // shared memory of an SM; the runtime's part of every CTA
+  static_assert(kPerSm * (kSmem + kReservedB) <= kSmB && kPerSmFused * (kSmemFused + kReservedB) <= kSmB,
+                "the CTAs that are to share an SM fit it");
 };
 
 template <typename Tile, int NW, int NS, bool kFused>

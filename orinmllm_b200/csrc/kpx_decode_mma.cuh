@@ -119,6 +119,7 @@ struct MmaTile {
   // at a time over the banks
   static constexpr int kRowStride = kRowB + 16;
   static constexpr bool kTensorMaps = true;
+  static constexpr int kWidestForm = 8;  // warps of the cluster form that has an SM to itself
   float by;           // what a product with the query rows is multiplied by to be a score (set by scale_q)
   uint32_t qa[8][2];  // A fragments: k step s holds d = 16s + 2t, +1 and 16s + 8 + 2t, +1 of head g
   float acc[16][4];   // d = 8 * tile + 2t, +1 of head g: [0..1] the P_hi part, [2..3] the P_lo part

@@ -20,3 +20,10 @@ def test_a_device_value_is_worked_out_once(tmp_path):
     subprocess.run(["g++", "-O2", "-std=c++17", "-pthread", "-I", b.CSRC, "-o", exe, CPP / "test_per_device.cpp"], check=True)
     run = subprocess.run([exe], capture_output=True, text=True)
     assert run.returncode == 0, run.stdout
+
+
+def test_narrow_cluster_forms_share_an_sm(tmp_path):
+    exe = tmp_path / "cluster_forms"
+    subprocess.run([b._nvcc(), *b.NVCC_FLAGS, "-o", exe, CPP / "test_cluster_forms.cu", "-lcuda"], check=True)
+    run = subprocess.run([exe], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout
