@@ -593,13 +593,17 @@ __global__ void __launch_bounds__(kThreads, 1)
           const int what = p.withhold_cta >> 16;
           const bool fault = p.withhold_cta >= 0 && int(blockIdx.x) == (p.withhold_cta & 0xffff) && u == u_first &&
                              jt == d.tile0 + (what == 2 ? 1 : 0) && values == (what == 1);
-          if (again) ok = wait(values ? bars.pv_done[buf.at] : bars.s_full[buf.at], buf.parity ^ 1u);
+          // A barrier is waited for only by a role that its next phase cannot do without: one that it can outrun would
+          // find the parity turned twice and wait for ever.  CTA 1 has no keys in a last tile of up to 64, whose
+          // scores CTA 0's keys alone let go.  (Without this wait it is never more than a phase ahead: only the last
+          // tile of a unit is such a tile, and a unit is begun when the rows of the one before the last have left.)
+          const int here = nblk - rank * (kTileBlocks / 2);  // blocks of this CTA's half of K that exist
+          if (again && (values || here > 0)) ok = wait(values ? bars.pv_done[buf.at] : bars.s_full[buf.at], buf.parity ^ 1u);
           if (!ok) break;
           if (!values) {
             int blk[kTileBlocks / 2];
 #pragma unroll
             for (int i = 0; i < kTileBlocks / 2; ++i) blk[i] = __shfl_sync(0xffffffffu, id, rank * (kTileBlocks / 2) + i);
-            const int here = nblk - rank * (kTileBlocks / 2);  // blocks of this CTA's half that exist
             if (elect_one()) {
               uint64_t* bar = &bars.scores_go[buf.at];
               if (rank == 0) mbar_arrive_expect_tx(bar, uint32_t(nblk) * (kBS * kD * 2));
