@@ -38,12 +38,13 @@
 #include <vector>
 
 #include "kpx_once.h"
+#include "kpx_prefill_plan.h"
 #include "kpx_tma.cuh"
 
 namespace kpx {
 namespace {
 
-constexpr int kD = 128, kBS = 16, kTile = 128;
+constexpr int kD = 128, kBS = 16;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr int kQItemB = kTile * kD * 2;     // an item's rows: two slabs of 64 elements, 128 bytes a row
 constexpr int kQSlabB = kQItemB / 2;
@@ -51,21 +52,9 @@ constexpr int kHalfB = kTile * kD;          // a CTA's half of a K or V tile
 constexpr int kKSlabB = kHalfB / 2;         // 64 keys x 64 elements
 constexpr int kBufs = 3;  // of scores / weights in tensor memory, and of K and of V in shared memory
 
-// A unit: `ntok` tokens of sequence `seq` from query row `tok0` on (cache position pos0), query heads
-// group * group_heads and on, and its share [tile0, tile1) of the key tiles.  Item 0 has the first
-// `tokens an item`, item 1 the rest; where they fit one item, it is item 1.  part >= 0: the keys were
-// cut, and the unnormalised rows go to that slot.
-struct alignas(16) Unit {
-  int32_t seq, group, tok0, ntok, pos0, tile0, tile1, part;
-};
-// A unit whose keys were cut: `parts` slots from slot0 on.
-struct alignas(16) Merge {
-  int32_t group, tok0, ntok, slot0, parts, pad[3];
-};
 // A slot holds, for both items of a unit, 128 rows of O, then 128 maxima and 128 sums (floats).
 constexpr int64_t kPartItemFloats = int64_t(kTile) * (kD + 2);
 constexpr int64_t kPartSlotFloats = 2 * kPartItemFloats;
-constexpr int kMaxPartSlots = 320;
 constexpr int kMaxClusters = 96;
 // The work list of a call travels as a kernel parameter where it fits (a copy of a list on the stream
 // is a few microseconds on the host and on the GPU); beyond kInlineUnits it lies in the work area.
@@ -74,7 +63,6 @@ struct UnitList {
   uint16_t start[kMaxClusters + 1];  // units start[c] .. start[c + 1] - 1 are cluster c's
   Unit unit[kInlineUnits];
 };
-constexpr int kMaxMerges = kMaxPartSlots / 2;
 struct MergeList {
   Merge merge[kMaxMerges];
 };
@@ -952,7 +940,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // Output rows of a unit whose keys were cut into parts: out = sum_p 2^(m_p - M) O_p / sum_p 2^(m_p - M) l_p.
 // blockIdx.x = unit, blockIdx.y = item and group of 8 rows; a warp per row, four elements a lane.  Bound by the
 // chain of loads: maxima and sums in one trip, then all parts' rows in one.
-constexpr int kMergeWarps = 8, kMaxParts = 8;
+constexpr int kMergeWarps = 8;
 template <typename T>
 __global__ void __launch_bounds__(32 * kMergeWarps)
     prefill_merge_kernel(T* __restrict__ out, const float* __restrict__ partials, int num_q_heads, int group_heads,
@@ -1025,74 +1013,6 @@ int g_prefill_split = -1;
 uint32_t g_prefill_wait_limit = kWaitLimit;
 int g_prefill_withhold_cta = -1;
 
-namespace {
-
-// Unit indexes, longest first (units of a length in their order).  Lengths are counted, not compared: at most
-// a few hundred key tiles, and a call makes its list while the GPU waits.
-std::vector<int32_t> longest_first(const std::vector<Unit>& units) {
-  int most = 0;
-  for (const Unit& d : units) most = std::max(most, d.tile1 - d.tile0);
-  std::vector<int32_t> at(size_t(most) + 2, 0), order(units.size(), 0);
-  for (const Unit& d : units) ++at[size_t(most - (d.tile1 - d.tile0)) + 1];
-  for (int i = 0; i <= most; ++i) at[size_t(i) + 1] += at[size_t(i)];
-  for (size_t i = 0; i < units.size(); ++i) order[size_t(at[size_t(most - (units[i].tile1 - units[i].tile0))]++)] = int32_t(i);
-  return order;
-}
-
-// Units dealt to `clusters` clusters, longest first to the least loaded; fills order (unit indexes,
-// cluster by cluster) and start.  Returns the largest load.  A unit costs its tiles and kUnitCost.
-constexpr int kUnitCost = 1;
-int deal_units(const std::vector<Unit>& units, int clusters, std::vector<int32_t>& order, std::vector<int32_t>& start) {
-  const int n = int(units.size());
-  const std::vector<int32_t> by_length = longest_first(units);
-  std::vector<int32_t> owner(size_t(n), 0), load(size_t(clusters), 0), heap(size_t(clusters), 0);
-  auto cost = [&](int i) { return units[size_t(i)].tile1 - units[size_t(i)].tile0 + kUnitCost; };
-  for (int c = 0; c < clusters; ++c) heap[size_t(c)] = c;  // a heap with the least loaded on top (ties: lowest index)
-  auto less = [&](int a, int b) { return load[size_t(a)] != load[size_t(b)] ? load[size_t(a)] < load[size_t(b)] : a < b; };
-  start.assign(size_t(clusters) + 1, 0);
-  int longest = 0;
-  for (int i : by_length) {
-    const int c = heap[0];
-    owner[size_t(i)] = c;
-    load[size_t(c)] += cost(i);
-    longest = std::max(longest, load[size_t(c)]);
-    ++start[size_t(c) + 1];
-    for (int at = 0;;) {  // sift down
-      int child = 2 * at + 1;
-      if (child >= clusters) break;
-      if (child + 1 < clusters && less(heap[size_t(child) + 1], heap[size_t(child)])) ++child;
-      if (!less(heap[size_t(child)], heap[size_t(at)])) break;
-      std::swap(heap[size_t(at)], heap[size_t(child)]);
-      at = child;
-    }
-  }
-  for (int c = 0; c < clusters; ++c) start[size_t(c) + 1] += start[size_t(c)];
-  std::vector<int32_t> at(start.begin(), start.end() - 1);
-  order.assign(size_t(n), 0);
-  for (int i : by_length) order[size_t(at[size_t(owner[size_t(i)])]++)] = i;
-  return longest;
-}
-
-// Cuts unit d along its keys into k parts, slots from `slot` on.
-void cut_unit(const Unit& d, int k, int& slot, std::vector<Unit>& units, std::vector<Merge>& merges) {
-  const int tiles = d.tile1 - d.tile0;
-  k = std::min(k, tiles);
-  if (k < 2 || slot + k > kMaxPartSlots || int(merges.size()) >= kMaxMerges) {
-    units.push_back(d);
-    return;
-  }
-  merges.push_back(Merge{d.group, d.tok0, d.ntok, slot, k, {0, 0, 0}});
-  for (int j = 0; j < k; ++j) {
-    Unit c = d;
-    c.tile0 = d.tile0 + int(int64_t(tiles) * j / k);
-    c.tile1 = d.tile0 + int(int64_t(tiles) * (j + 1) / k);
-    c.part = slot++;
-    units.push_back(c);
-  }
-}
-
-}  // namespace
-
 // Host side: work list, tensor maps, launch.  Returns KPX_ERR_UNIMPLEMENTED when the layout, dtype or scale
 // is outside this path so that the caller can fall back to the streaming path.
 int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool, const kpx_kv_layout* layout,
@@ -1112,90 +1032,17 @@ int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool,
   const int head_groups = kv_mul / group_heads, groups = kv_heads * head_groups;
   const int item_tokens = kTile / group_heads;
   const int clusters = std::min(std::max(device_info().sm_count / 2, 1), kMaxClusters);
-  std::vector<Unit> units;
-  units.reserve(size_t(total_q / (2 * item_tokens) + batch) * size_t(groups));
-  int64_t tiles = 0;
-  int longest = 0;
-  for (int32_t b = 0; b < batch; ++b) {
-    const int32_t n = cu_q_lens_host[b + 1] - cu_q_lens_host[b];
-    for (int32_t t = 0; t < n; t += 2 * item_tokens) {
-      const int ntok = std::min(2 * item_tokens, n - t), pos = start_pos_host[b] + t, end = (pos + ntok - 1) / kTile + 1;
-      for (int32_t h = 0; h < groups; ++h) units.push_back(Unit{b, h, cu_q_lens_host[b] + t, ntok, pos, 0, end, -1});
-      tiles += int64_t(end) * groups;
-      longest = std::max(longest, end);
-    }
-  }
+  std::vector<Unit> units = whole_units(cu_q_lens_host, start_pos_host, batch, groups, item_tokens);
   if (units.empty()) return KPX_OK;
-  std::vector<int32_t> order, start;
-  std::vector<Merge> merges;
-  const int n = int(units.size());
-  if (g_prefill_split >= 2) {  // test knob: always cut
-    std::vector<Unit> parts;
-    int slot = 0;
-    for (const Unit& d : units) cut_unit(d, std::min(g_prefill_split, 4), slot, parts, merges);
-    units.swap(parts);
-    deal_units(units, clusters, order, start);
-  } else {
-    const int load = deal_units(units, clusters, order, start);
-    // Cut along the keys where whole units leave many clusters idle for long: a part costs its rows
-    // written and read in fp32 and the call a second launch, together about kMergeCost tiles.
-    constexpr int kMergeCost = 4;
-    const int64_t even = (tiles + int64_t(n) * kUnitCost + clusters - 1) / clusters;
-    const int idle = load - int(even);
-    if (g_prefill_split != 0 && idle > kMergeCost && idle * int64_t(8) > even) {
-      std::vector<Unit> parts;
-      parts.reserve(units.size() + kMaxPartSlots);
-      int slot = 0;
-      if (longest > even) {
-        // A few long units: no part longer than a k-th of the longest, k by the rounds that the parts make.  (Cut to
-        // an even share instead, whatever the rounds: 512 tokens behind 3584, 32/8 heads, 64 units on 74 clusters, 51 us
-        // against 42; 256 behind 8192, 28/4, 71 against 59; 256 behind 3840, 32/8, 41 against 36.)
-        int cap = 0, best = load;
-        for (int k = 2; k <= kMaxParts; ++k) {
-          const int c = (longest + k - 1) / k;
-          int64_t count = 0;
-          for (const Unit& d : units) count += (d.tile1 + c - 1) / c;
-          const int64_t rounds = (count + clusters - 1) / clusters, mean = (tiles + count * kUnitCost + count - 1) / count;
-          const int cost = int(std::max<int64_t>(c + kUnitCost, rounds * mean)) + kMergeCost;
-          if (cost < best) {
-            best = cost;
-            cap = c;
-          }
-        }
-        if (cap > 0)
-          for (const Unit& d : units) cut_unit(d, std::min(kMaxParts, (d.tile1 + cap - 1) / cap), slot, parts, merges);
-      } else {  // many units of like length and a thin last round: the shortest, a round's remainder, are cut
-        const int rest = n % clusters;
-        const std::vector<int32_t> by_length = longest_first(units);
-        const int t = units[size_t(by_length[size_t(n - 1)])].tile1 + 1;
-        int k = 1, best = (t + kUnitCost) * 8;  // eighths of a tile
-        for (int c = 2; c <= kMaxParts && rest > 0; ++c) {
-          const int rounds = (rest * c + clusters - 1) / clusters;
-          const int cost = rounds * (t * 8 / c + 8 * kUnitCost) + 8 * kMergeCost;
-          if (cost < best) {
-            best = cost;
-            k = c;
-          }
-        }
-        if (k > 1) {
-          for (int i = 0; i < n - rest; ++i) parts.push_back(units[size_t(by_length[size_t(i)])]);
-          for (int i = n - rest; i < n; ++i) cut_unit(units[size_t(by_length[size_t(i)])], k, slot, parts, merges);
-        }
-      }
-      if (!merges.empty()) {
-        units.swap(parts);
-        deal_units(units, clusters, order, start);
-      }
-    }
-  }
+  const WorkList work = plan_units(std::move(units), clusters, g_prefill_split);
   // clusters with work
   int used = clusters;
-  while (used > 1 && start[size_t(used)] == start[size_t(used) - 1]) --used;
+  while (used > 1 && work.start[size_t(used)] == work.start[size_t(used) - 1]) --used;
   // layout of the area: [starts][units] (lists that do not fit a parameter), [part slots]
-  const bool inline_list = int(units.size()) <= kInlineUnits;
+  const bool inline_list = int(work.units.size()) <= kInlineUnits;
   const int64_t start_bytes = inline_list ? 0 : align256(int64_t(clusters + 1) * 4);
-  const int64_t unit_bytes = inline_list ? 0 : align256(int64_t(units.size()) * int64_t(sizeof(Unit)));
-  const int64_t slot_bytes = merges.empty() ? 0 : int64_t(kMaxPartSlots) * kPartSlotFloats * int64_t(sizeof(float));
+  const int64_t unit_bytes = inline_list ? 0 : align256(int64_t(work.units.size()) * int64_t(sizeof(Unit)));
+  const int64_t slot_bytes = work.merges.empty() ? 0 : int64_t(kMaxPartSlots) * kPartSlotFloats * int64_t(sizeof(float));
   if (start_bytes + unit_bytes + slot_bytes > tile_area_bytes) return KPX_ERR_WORKSPACE_TOO_SMALL;
 
   CUtensorMap map_q, map_k, map_v, map_out;
@@ -1223,14 +1070,14 @@ int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool,
   UnitList list;
   PrefillParams p;
   if (inline_list) {
-    for (int c = 0; c <= clusters; ++c) list.start[c] = uint16_t(start[size_t(c)]);
-    for (size_t i = 0; i < units.size(); ++i) list.unit[i] = units[size_t(order[i])];
+    for (int c = 0; c <= clusters; ++c) list.start[c] = uint16_t(work.start[size_t(c)]);
+    for (size_t i = 0; i < work.units.size(); ++i) list.unit[i] = work.units[size_t(work.order[i])];
     p.starts = nullptr;
     p.units = nullptr;
   } else {
-    std::vector<Unit> in_order(units.size());
-    for (size_t i = 0; i < units.size(); ++i) in_order[i] = units[size_t(order[i])];
-    KPX_CUDA_TRY(cudaMemcpyAsync(area, start.data(), start.size() * 4, cudaMemcpyHostToDevice, stream));
+    std::vector<Unit> in_order(work.units.size());
+    for (size_t i = 0; i < work.units.size(); ++i) in_order[i] = work.units[size_t(work.order[i])];
+    KPX_CUDA_TRY(cudaMemcpyAsync(area, work.start.data(), work.start.size() * 4, cudaMemcpyHostToDevice, stream));
     KPX_CUDA_TRY(cudaMemcpyAsync(area + start_bytes, in_order.data(), in_order.size() * sizeof(Unit),
                                  cudaMemcpyHostToDevice, stream));
     p.starts = reinterpret_cast<const int32_t*>(area);
@@ -1259,10 +1106,10 @@ int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool,
   };
   const int rc = layout->dtype == KPX_F16 ? launch(prefill_tc_kernel<__half>, ready_f16)
                                           : launch(prefill_tc_kernel<__nv_bfloat16>, ready_bf16);
-  if (rc != KPX_OK || merges.empty()) return rc;
+  if (rc != KPX_OK || work.merges.empty()) return rc;
   MergeList mlist;
-  std::copy(merges.begin(), merges.end(), mlist.merge);
-  const dim3 mgrid(unsigned(merges.size()), 2 * (kTile / kMergeWarps)), mblock(32 * kMergeWarps);
+  std::copy(work.merges.begin(), work.merges.end(), mlist.merge);
+  const dim3 mgrid(unsigned(work.merges.size()), 2 * (kTile / kMergeWarps)), mblock(32 * kMergeWarps);
   return layout->dtype == KPX_F16
              ? launch_chained(prefill_merge_kernel<__half>, mgrid, mblock, 0, stream, static_cast<__half*>(out), p.partials,
                               num_q_heads, group_heads, item_tokens, mlist)

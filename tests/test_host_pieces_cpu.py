@@ -27,3 +27,10 @@ def test_narrow_cluster_forms_share_an_sm(tmp_path):
     subprocess.run([b._nvcc(), *b.NVCC_FLAGS, "-o", exe, CPP / "test_cluster_forms.cu", "-lcuda"], check=True)
     run = subprocess.run([exe], capture_output=True, text=True)
     assert run.returncode == 0, run.stdout
+
+
+def test_prefill_work_lists(tmp_path):
+    exe = tmp_path / "prefill_plan"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-I", b.CSRC, "-o", exe, CPP / "test_prefill_plan.cpp"], check=True)
+    run = subprocess.run([exe], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout
