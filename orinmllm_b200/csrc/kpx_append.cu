@@ -1,10 +1,11 @@
 // K/V append into the block pool, RoPE(+append), sin/cos tables, copy-on-write
 // block copy and block refcount updates.  All of these are pure data movement
-// (or element-wise fp32 math) bound by HBM bandwidth: 128-bit accesses,
-// grid-stride loops sized from the SM count.
-#include <type_traits>
+// (or element-wise fp32 math) bound by HBM bandwidth: 128-bit accesses.  Grids are
+// sized from the SM count, by token where a CTA's threads share what a token needs.
+#include <algorithm>
 
 #include "kpx_common.cuh"
+#include "kpx_rope_form.h"
 
 namespace kpx {
 namespace {
@@ -102,9 +103,10 @@ append_kernel(uint8_t* __restrict__ k_pool, uint8_t* __restrict__ v_pool,
 // of one head of one token, i.e. one 16-byte vector at j and one at j+head_size/2.
 // Bound by the chain position -> sin / cos -> store up to about a hundred tokens, by how many such chains an SM
 // holds beyond.  kVec: sin, cos and norm weights lie on 16-byte boundaries and are fetched four floats at a time,
-// all before the norm, which takes their trip off the chain and costs registers (80 instead of 48).
-// Measured and dropped: two or four heads of a token per thread (fewer chains held: norm, 2048 tokens 15.3 / 18.7
-// against 14.8 us), kVec in 64 or 48 registers (spills: 19.1 / 24.7).
+// all before the norm, which takes their trip off the chain and costs registers (80 instead of 48; fp32 52 instead
+// of 40).  Which form a call takes: kpx_rope_form.h.
+// Measured and dropped, when this was the form of 2048 tokens too: two or four heads of a token per thread (fewer
+// chains held: 15.3 / 18.7 against 14.8 us), kVec in 64 or 48 registers (spills: 19.1 / 24.7).
 template <int kN>
 __device__ __forceinline__ void load4(const float* p, float (&f)[kN]) {
 #pragma unroll
@@ -367,8 +369,9 @@ rope_rows_kernel(T* __restrict__ q, T* __restrict__ k, const T* __restrict__ v, 
 // (which head, which vector, K or V) is then fixed for the whole launch and is decoded once;
 // per token there is one slot fetch and one 64-bit base address.  append_kernel above (one flat
 // index per item, decoded anew each time) remains the fallback for wider tokens: it spends
-// about half of the SM's issue slots on index arithmetic at 16 bytes per item.  (The same
-// form of the RoPE kernel measured no faster than the flat one and is not kept.)
+// about half of the SM's issue slots on index arithmetic at 16 bytes per item.
+// (Threads with fixed roles that walk over tokens gave the RoPE kernel nothing; what gave something there is
+// sharing a token's tables within a CTA, rope_rows_kernel.)
 __device__ __forceinline__ int64_t slot_base_bytes(const LayoutDev& L, int64_t slot) {
   int64_t blk, off;
   if (uint64_t(slot) < 0x80000000ull) {
@@ -524,11 +527,10 @@ inline int grid_for(int64_t work_items, int threads) {
   return int(blocks);
 }
 
-// Grid of a grid-stride kernel capped at exactly what the SMs hold at once (from the occupancy
-// calculator, looked up once per kernel): a cap above that runs the surplus CTAs as a second,
-// partly filled wave.
+// CTAs that the SMs hold at once (from the occupancy calculator, looked up once per kernel).  The grid of a
+// grid-stride kernel is capped at exactly that: a cap above it runs the surplus CTAs as a second, partly filled wave.
 template <auto kernel>
-inline int resident_grid_for(int64_t work_items, int threads) {
+inline int64_t resident_ctas(int threads) {
   static int per_sm = 0;
   if (per_sm == 0) {
     int n = 0;
@@ -536,10 +538,7 @@ inline int resident_grid_for(int64_t work_items, int threads) {
     per_sm = n;
   }
   const DeviceInfo& di = device_info();
-  int64_t blocks = (work_items + threads - 1) / threads;
-  const int64_t cap = int64_t(di.sm_count > 0 ? di.sm_count : 148) * per_sm;
-  if (blocks > cap) blocks = cap;
-  return int(blocks < 1 ? 1 : blocks);
+  return int64_t(di.sm_count > 0 ? di.sm_count : 148) * per_sm;
 }
 
 // Grid of a token-walking kernel: one CTA per token up to what the SMs hold at once (from the
@@ -590,15 +589,6 @@ extern "C" int kpx_append(void* k_pool, void* v_pool, const kpx_kv_layout* layou
   return cuda_status(cudaGetLastError());
 }
 
-// Up to this many threads the form that fetches tables and weights early is launched where there is a norm.
-// norm + RoPE + append, fp16 32/8 heads, us, that form / the other: 1 token 1.96 / 2.37, 64 2.35 / 2.65, 256
-// 4.00 / 4.52, 777 7.15 / 7.40, 2048 (0.9 million threads) 14.4 / 14.8, 16384 113 / 98.  Without a norm there is no
-// more to fetch than the chain brings anyway: bf16 28/4 1.89 / 1.81, 2.14 / 2.06, fp32 1.74 / 1.66, 1.99 / 1.93.
-constexpr int64_t kEarlyTables = 1000000;
-// From kRowsFrom tokens on 16-bit rows of 128 take rope_rows_kernel (256 tokens: 4.4 / 2.8 us against 3.9 / 2.7 of the
-// flat forms; 512: 5.0 / 3.1 against 5.3 / 3.8), from kRowsPairs on with two tokens a CTA (777: 7.0 / 4.4 against 6.2 /
-// 3.9 with one; 2048: 10.4 / 6.3 against 11.5 / 7.3).
-constexpr int kRowsFrom = 400, kRowsPairs = 1400;
 template <typename T>
 static int launch_rope(void* q, void* k, const void* v, int32_t q_heads, const int32_t* positions,
                        int32_t pos_base, const float* sin_cache, const float* cos_cache, void* k_pool, void* v_pool,
@@ -614,28 +604,31 @@ static int launch_rope(void* q, void* k, const void* v, int32_t q_heads, const i
   const int vvecs = (v && v_pool) ? L.num_kv_heads * L.head_size / E : 0;
   if (heads * groups + vvecs == 0) return KPX_OK;
   const int64_t work = int64_t(num_tokens) * (heads * groups + vvecs);
-  auto launch = [&](auto early) {
-    constexpr auto kernel = rope_append_kernel<T, decltype(early)::value>;
-    const int threads = 256;
-    return launch_chained(kernel, dim3(resident_grid_for<kernel>(work, threads)), dim3(threads), 0, stream, static_cast<T*>(q),
+  auto launch = [&](auto kernel, int64_t grid, int threads) {
+    return launch_chained(kernel, dim3(unsigned(grid)), dim3(unsigned(threads)), 0, stream, static_cast<T*>(q),
                           static_cast<T*>(k), static_cast<const T*>(v), q_heads, positions, pos_base, sin_cache, cos_cache,
                           static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool), slot_mapping, num_tokens, L, q_norm_w,
                           k_norm_w, norm_eps);
   };
+  constexpr auto flat = rope_append_kernel<T, false>, early = rope_append_kernel<T, true>;
+  const int threads = 256;
+  RopeCall call;
+  call.elt_bytes = sizeof(T);
+  call.head_size = L.head_size;
+  call.tokens = num_tokens;
+  call.norm = q_norm_w || k_norm_w;
+  call.aligned = ((reinterpret_cast<uintptr_t>(sin_cache) | reinterpret_cast<uintptr_t>(cos_cache) |
+                   reinterpret_cast<uintptr_t>(q_norm_w) | reinterpret_cast<uintptr_t>(k_norm_w)) & 15) == 0;
+  call.ctas = (work + threads - 1) / threads;
+  call.flat_fit = resident_ctas<flat>(threads);
+  call.early_fit = resident_ctas<early>(threads);
+  const RopeForm form = rope_form(call);
   if constexpr (sizeof(T) == 2) {
-    auto launch_rows = [&](auto kernel, int tokens) {
-      return launch_chained(kernel, dim3(unsigned((int64_t(num_tokens) + tokens - 1) / tokens)), dim3(kRowsThreads), 0, stream,
-                            static_cast<T*>(q), static_cast<T*>(k), static_cast<const T*>(v), q_heads, positions, pos_base,
-                            sin_cache, cos_cache, static_cast<uint8_t*>(k_pool), static_cast<uint8_t*>(v_pool), slot_mapping,
-                            num_tokens, L, q_norm_w, k_norm_w, norm_eps);
-    };
-    if (L.head_size == 128 && num_tokens >= kRowsFrom)
-      return num_tokens < kRowsPairs ? launch_rows(rope_rows_kernel<T, 1>, 1) : launch_rows(rope_rows_kernel<T, 2>, 2);
+    if (form == RopeForm::kOneToken) return launch(rope_rows_kernel<T, 1>, num_tokens, kRowsThreads);
+    if (form == RopeForm::kTwoTokens) return launch(rope_rows_kernel<T, 2>, (int64_t(num_tokens) + 1) / 2, kRowsThreads);
   }
-  const bool aligned = ((reinterpret_cast<uintptr_t>(sin_cache) | reinterpret_cast<uintptr_t>(cos_cache) |
-                         reinterpret_cast<uintptr_t>(q_norm_w) | reinterpret_cast<uintptr_t>(k_norm_w)) & 15) == 0;
-  if (aligned && (q_norm_w || k_norm_w) && work <= kEarlyTables) return launch(std::true_type());
-  return launch(std::false_type());
+  if (form == RopeForm::kEarlyTables) return launch(early, std::min(call.ctas, call.early_fit), threads);
+  return launch(flat, std::min(call.ctas, call.flat_fit), threads);
 }
 
 extern "C" int kpx_rope_append(void* q, void* k, const void* v, int32_t q_heads,

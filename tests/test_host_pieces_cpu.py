@@ -34,3 +34,10 @@ def test_prefill_work_lists(tmp_path):
     subprocess.run(["g++", "-O2", "-std=c++17", "-I", b.CSRC, "-o", exe, CPP / "test_prefill_plan.cpp"], check=True)
     run = subprocess.run([exe], capture_output=True, text=True)
     assert run.returncode == 0, run.stdout
+
+
+def test_form_of_the_rope_kernel(tmp_path):
+    exe = tmp_path / "rope_form"
+    subprocess.run(["g++", "-O2", "-std=c++17", "-I", b.CSRC, "-o", exe, CPP / "test_rope_form.cpp"], check=True)
+    run = subprocess.run([exe], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout
