@@ -339,6 +339,46 @@ __device__ __noinline__ void stage_new_token(const T* q_kv_group, int hg, int kv
   }
 }
 
+// The same, rows one after the other: for the fp32 kernel along the line of blocks, which has no registers to spare.
+// With all rows in one trip it was the slower kernel (fused, 10 sequences of 1500..3000 tokens, 12/2 heads 32.0 -> 33.6
+// us, 16/2 30.6 -> 32.6; of 400..1500, 32/8 24.5 -> 25.7; so it was with turns of rows in registers).
+template <typename T, int QH, int kRowStride>
+__device__ __noinline__ void stage_new_token_in_turns(const T* q_kv_group, int hg, int kv_mul, const T* k_row,
+                                                      const uint8_t* v_row, bool with_kv, const float* sin_row,
+                                                      const float* cos_row, const int32_t* table_entry,
+                                                      int identity_id, uint8_t* stage, int lane) {
+  constexpr int E = Elt<T>::kPer16B;
+  constexpr int G = kD / 2 / E;  // 16-byte pair groups per row
+  constexpr int kRowB = kD * int(sizeof(T));
+  const int rows = QH + (with_kv ? 1 : 0);
+  for (int task = lane; task < rows * G; task += 32) {
+    const int r = task / G, g = task - r * G;
+    const int hq = hg * QH + r;
+    const T* src = r < QH ? q_kv_group + (hq < kv_mul ? hq : 0) * kD : k_row;
+    float lo[E], hi[E];
+    Elt<T>::unpack(__ldg(reinterpret_cast<const uint4*>(src + g * E)), lo);
+    Elt<T>::unpack(__ldg(reinterpret_cast<const uint4*>(src + kD / 2 + g * E)), hi);
+    __align__(16) T lo_out[E];
+    __align__(16) T hi_out[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      const float sn = __ldg(sin_row + 2 * (g * E + e)), cs = __ldg(cos_row + 2 * (g * E + e));
+      lo_out[e] = Elt<T>::from_float(__fsub_rn(__fmul_rn(lo[e], cs), __fmul_rn(hi[e], sn)));
+      hi_out[e] = Elt<T>::from_float(__fadd_rn(__fmul_rn(lo[e], sn), __fmul_rn(hi[e], cs)));
+    }
+    uint8_t* dst = stage + r * kRowStride;
+    *reinterpret_cast<uint4*>(dst + g * 16) = *reinterpret_cast<const uint4*>(lo_out);
+    *reinterpret_cast<uint4*>(dst + kRowB / 2 + g * 16) = *reinterpret_cast<const uint4*>(hi_out);
+  }
+  if (with_kv) {
+    for (int task = lane; task < kRowB / 16; task += 32)
+      *reinterpret_cast<uint4*>(stage + (QH + 1) * kRowStride + task * 16) =
+          __ldg(reinterpret_cast<const uint4*>(v_row) + task);
+    if (lane == 0)
+      *reinterpret_cast<int32_t*>(stage + (QH + 2) * kRowStride) = table_entry ? __ldg(table_entry) : identity_id;
+  }
+}
+
 // kSmall: the form launched when the host can tell from the batch size and the table width that
 // the launch has only a few blocks per warp (a short batch, or one KV head of one long
 // sequence).  It cuts the line into fewer, longer ranges: every piece of a cut item costs a
@@ -538,7 +578,7 @@ paged_decode_kernel(const DecodeParams p) {
       const int seg = min(blocks_left, cur.nblk - cur.blk);
       const bool ends_item = cur.blk + seg == cur.nblk;
       __syncwarp();  // the previous item's readers of the staging area are done
-      stage_new_token<T, QH, kD * C::kEltB>(
+      stage_new_token_in_turns<T, QH, kD * C::kEltB>(
           qrow + int64_t(cur.kvh) * p.kv_mul * kD, hg, p.kv_mul,
           static_cast<const T*>(p.k_new) + (int64_t(cur.b) * p.num_kv_heads + cur.kvh) * kD,
           static_cast<const uint8_t*>(p.v_new) + (int64_t(cur.b) * p.num_kv_heads + cur.kvh) * (kD * C::kEltB),
