@@ -35,6 +35,7 @@
 // Every wait is bounded; a role that gives up raises its CTA's flag, the other CTA runs out of its own
 // waits, tensor memory is freed on every path and the workspace status word is raised.
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "kpx_once.h"
@@ -56,12 +57,18 @@ constexpr int kBufs = 3;  // of scores / weights in tensor memory, and of K and 
 constexpr int64_t kPartItemFloats = int64_t(kTile) * (kD + 2);
 constexpr int64_t kPartSlotFloats = 2 * kPartItemFloats;
 constexpr int kMaxClusters = 96;
-// The work list of a call travels as a kernel parameter where it fits (a copy of a list on the stream
-// is a few microseconds on the host and on the GPU); beyond kInlineUnits it lies in the work area.
-constexpr int kInlineUnits = 352;
+// The work list of a call travels as a kernel parameter where it fits.  A copy of it on the stream is a few
+// microseconds on the host and on the GPU, keeps the launch from being chained, and reads a list that is gone when a
+// captured graph is replayed.  kInlineUnits is what the 32764 bytes of a kernel's parameters hold beside the rest;
+// beyond it the list lies in the work area.  All parameters are copied with every launch, so lists of up to kFewUnits
+// go in shorter ones (a call of 8/8 heads, 8 x 100 tokens 9.1 us, 9.5 with the long list; 777 tokens, 32/8 15.0 / 15.1).
+// Copied / as a parameter, us: 400 units (8/8 heads, 50 x 64 tokens behind 100) 40.3 / 34.9, 512 (32/8, 64 x 16) 34.0 /
+// 27.7, (32/32, 16 x 100 behind 50) 46.4 / 40.5, 640 (8/8, 80 x 64 behind 100) 57.7 / 51.3.
+constexpr int kFewUnits = 352, kInlineUnits = 960;
+template <int kUnits>
 struct UnitList {
   uint16_t start[kMaxClusters + 1];  // units start[c] .. start[c + 1] - 1 are cluster c's
-  Unit unit[kInlineUnits];
+  Unit unit[kUnits];
 };
 struct MergeList {
   Merge merge[kMaxMerges];
@@ -86,6 +93,9 @@ struct PrefillParams {
   uint32_t wait_limit;
   int32_t withhold_cta;
 };
+
+static_assert(sizeof(PrefillParams) + 64 + 4 * sizeof(CUtensorMap) + 64 + sizeof(UnitList<kInlineUnits>) <= 32764,
+              "a kernel's parameters");
 
 // ---- PTX wrappers -----------------------------------------------------------------------
 __device__ __forceinline__ uint32_t cluster_rank() {
@@ -408,7 +418,9 @@ constexpr float kLazyMax = 8.f;
 
 constexpr int kPvWarp = 8, kKeyWarp = 9, kValueWarp = 10, kScoresWarp = 11;
 // Launched with 168 registers a thread (12 warps x 32 x 168 = 64512); the softmax groups then take 208 and the
-// other four warps keep 88: 256 x 208 + 128 x 88 = 64512.
+// other four warps keep 88: 256 x 208 + 128 x 88 = 64512.  The compiler allots all roles the 168 of the launch and
+// spills 84 bytes in the softmax role, between its masked tiles and the rows' way out (none without that role, 12
+// without either of the two).
 constexpr int kThreads = 384;
 struct Bars {
   uint64_t v_here;           // a last tile of V has landed in this CTA
@@ -446,12 +458,12 @@ struct Ring {
   }
 };
 
-template <typename T>
+template <typename T, int kUnits>
 __global__ void __launch_bounds__(kThreads, 1)
     prefill_tc_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap map_q,
                       const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                       const __grid_constant__ CUtensorMap map_out,
-                      const __grid_constant__ UnitList list) {
+                      const __grid_constant__ UnitList<kUnits> list) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint8_t* sQ = smem;                     // this CTA's item of two units in turn
@@ -1067,11 +1079,8 @@ int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool,
       return KPX_ERR_UNIMPLEMENTED;
   }
   uint8_t* area = static_cast<uint8_t*>(tile_area);
-  UnitList list;
   PrefillParams p;
   if (inline_list) {
-    for (int c = 0; c <= clusters; ++c) list.start[c] = uint16_t(work.start[size_t(c)]);
-    for (size_t i = 0; i < work.units.size(); ++i) list.unit[i] = work.units[size_t(work.order[i])];
     p.starts = nullptr;
     p.units = nullptr;
   } else {
@@ -1097,15 +1106,25 @@ int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool,
   p.qscale = scale * kLog2e;
   p.wait_limit = g_prefill_wait_limit;
   p.withhold_cta = g_prefill_withhold_cta;
-  static PerDevice<Ready> ready_f16, ready_bf16;
-  auto launch = [&](auto kernel, PerDevice<Ready>& ready) -> int {
+  auto launch = [&](auto type, auto capacity) -> int {
+    constexpr int kUnits = decltype(capacity)::value;
+    constexpr auto kernel = prefill_tc_kernel<decltype(type), kUnits>;
+    static PerDevice<Ready> ready;
     const int rc = prepare_kernel(kernel, ready);
     if (rc != KPX_OK) return rc;
+    UnitList<kUnits> list;
+    if (inline_list) {
+      for (int c = 0; c <= clusters; ++c) list.start[c] = uint16_t(work.start[size_t(c)]);
+      for (size_t i = 0; i < work.units.size(); ++i) list.unit[i] = work.units[size_t(work.order[i])];
+    }
     return launch_chained_cluster(kernel, dim3(unsigned(2 * used)), dim3(kThreads), kSmemBytes, 2, stream, p, map_q, map_k,
                                   map_v, map_out, list);
   };
-  const int rc = layout->dtype == KPX_F16 ? launch(prefill_tc_kernel<__half>, ready_f16)
-                                          : launch(prefill_tc_kernel<__nv_bfloat16>, ready_bf16);
+  const bool few = !inline_list || int(work.units.size()) <= kFewUnits;
+  auto launch_as = [&](auto type) {
+    return few ? launch(type, std::integral_constant<int, kFewUnits>()) : launch(type, std::integral_constant<int, kInlineUnits>());
+  };
+  const int rc = layout->dtype == KPX_F16 ? launch_as(__half()) : launch_as(__nv_bfloat16());
   if (rc != KPX_OK || work.merges.empty()) return rc;
   MergeList mlist;
   std::copy(work.merges.begin(), work.merges.end(), mlist.merge);
