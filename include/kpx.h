@@ -258,10 +258,9 @@ KPX_API int kpx_workspace_status(void* workspace, void* stream);
  * its query i sits at position start_pos[b] + i and attends cache positions
  * 0 .. start_pos[b]+i.  cu_q_lens (int32 [batch+1]) and start_pos (int32 [batch])
  * are HOST arrays (they size the grid).
- * Capture: a 16-bit call of up to 960 units of work can be captured after a first call of its kind.  A unit is
- * 2 * (128 / n) tokens of a sequence and n = num_q_heads / num_kv_heads query heads (n up to 128; keys cut into parts
- * count a unit each, and parts are at most 320).  Longer calls, fp32 caches and other head and block sizes copy from
- * host memory that does not outlive the call: a graph must not hold them.
+ * Capture: calls of 16-bit caches in the paged layout with head size 128 and block size 16 can be captured, after a
+ * first call of their kind.  The others copy the two host arrays on the stream: a graph that holds such a call reads
+ * them at every replay, so they have to outlive it, unchanged.
  * Replaces batched_mha_kernel_cu (kuiper/source/op/kernels/cuda/mha_kernel.cuh:20-26),
  * flash_attention_prefill[_fp16]_cu, flash_attention2_prefill[_fp16]_cu (cuda/
  * flash_attention_kernel.cuh:27-42,71-86,139-174). */

@@ -35,6 +35,7 @@
 // Every wait is bounded; a role that gives up raises its CTA's flag, the other CTA runs out of its own
 // waits, tensor memory is freed on every path and the workspace status word is raised.
 #include <algorithm>
+#include <cstring>
 #include <type_traits>
 #include <vector>
 
@@ -57,10 +58,10 @@ constexpr int kBufs = 3;  // of scores / weights in tensor memory, and of K and 
 constexpr int64_t kPartItemFloats = int64_t(kTile) * (kD + 2);
 constexpr int64_t kPartSlotFloats = 2 * kPartItemFloats;
 constexpr int kMaxClusters = 96;
-// The work list of a call travels as a kernel parameter where it fits.  A copy of it on the stream is a few
-// microseconds on the host and on the GPU, keeps the launch from being chained, and reads a list that is gone when a
-// captured graph is replayed.  kInlineUnits is what the 32764 bytes of a kernel's parameters hold beside the rest;
-// beyond it the list lies in the work area.  All parameters are copied with every launch, so lists of up to kFewUnits
+// The work list of a call travels as a kernel parameter: a copy of it on the stream would be a few microseconds on the
+// host and on the GPU, keep the launch from being chained, and read a list that is gone when a captured graph is
+// replayed.  kInlineUnits is what the 32764 bytes of a kernel's parameters hold beside the rest; longer lists are
+// laid into the work area by launches of list_kernel, a parameter full at a time.  All parameters are copied with every launch, so lists of up to kFewUnits
 // go in shorter ones (a call of 8/8 heads, 8 x 100 tokens 9.1 us, 9.5 with the long list; 777 tokens, 32/8 15.0 / 15.1).
 // Copied / as a parameter, us: 400 units (8/8 heads, 50 x 64 tokens behind 100) 40.3 / 34.9, 512 (32/8, 64 x 16) 34.0 /
 // 27.7, (32/32, 16 x 100 behind 50) 46.4 / 40.5, 640 (8/8, 80 x 64 behind 100) 57.7 / 51.3.
@@ -69,6 +70,10 @@ template <int kUnits>
 struct UnitList {
   uint16_t start[kMaxClusters + 1];  // units start[c] .. start[c + 1] - 1 are cluster c's
   Unit unit[kUnits];
+};
+constexpr int kListPieces = 2000;  // of 16 bytes, in a parameter of list_kernel
+struct ListPieces {
+  uint4 piece[kListPieces];
 };
 struct MergeList {
   Merge merge[kMaxMerges];
@@ -1004,6 +1009,16 @@ __global__ void __launch_bounds__(32 * kMergeWarps)
       make_uint2(pack2<T>(acc.x * inv, acc.y * inv), pack2<T>(acc.z * inv, acc.w * inv));
 }
 
+// A stretch of a work list that is too long for the kernel's own parameters, into the work area.
+constexpr int kListThreads = 128;
+__global__ void __launch_bounds__(kListThreads)
+    list_kernel(uint4* __restrict__ dst, int count, const __grid_constant__ ListPieces list) {
+  const int64_t after_wait = grid_wait();
+  grid_release();
+  const int i = int(blockIdx.x) * kListThreads + int(threadIdx.x);
+  if (i < count) dst[i + after_wait] = list.piece[i];
+}
+
 struct Ready {};
 template <typename K>
 int prepare_kernel(K kernel, PerDevice<Ready>& done) {
@@ -1084,11 +1099,18 @@ int prefill_tc(void* out, const void* q, const void* k_pool, const void* v_pool,
     p.starts = nullptr;
     p.units = nullptr;
   } else {
-    std::vector<Unit> in_order(work.units.size());
-    for (size_t i = 0; i < work.units.size(); ++i) in_order[i] = work.units[size_t(work.order[i])];
-    KPX_CUDA_TRY(cudaMemcpyAsync(area, work.start.data(), work.start.size() * 4, cudaMemcpyHostToDevice, stream));
-    KPX_CUDA_TRY(cudaMemcpyAsync(area + start_bytes, in_order.data(), in_order.size() * sizeof(Unit),
-                                 cudaMemcpyHostToDevice, stream));
+    std::vector<uint4> image(size_t(start_bytes + unit_bytes) / sizeof(uint4));
+    std::memcpy(image.data(), work.start.data(), work.start.size() * 4);
+    Unit* units_at = reinterpret_cast<Unit*>(reinterpret_cast<uint8_t*>(image.data()) + start_bytes);
+    for (size_t i = 0; i < work.units.size(); ++i) std::memcpy(units_at + i, &work.units[size_t(work.order[i])], sizeof(Unit));
+    ListPieces pieces;
+    for (size_t at = 0; at < image.size(); at += kListPieces) {
+      const size_t count = std::min(image.size() - at, size_t(kListPieces));
+      std::memcpy(pieces.piece, image.data() + at, count * sizeof(uint4));
+      const int rc = launch_chained(list_kernel, dim3(unsigned((count + kListThreads - 1) / kListThreads)), dim3(kListThreads), 0,
+                                    stream, reinterpret_cast<uint4*>(area) + at, int(count), pieces);
+      if (rc != KPX_OK) return rc;
+    }
     p.starts = reinterpret_cast<const int32_t*>(area);
     p.units = reinterpret_cast<const Unit*>(area + start_bytes);
   }

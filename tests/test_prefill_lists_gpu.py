@@ -27,7 +27,7 @@ def _prompts(torch, capi, batch, tokens, start):
     return q, ws, call
 
 
-@pytest.mark.parametrize("batch", [44, 45, 120, 121])  # 352, 360, 960 and 968 units
+@pytest.mark.parametrize("batch", [44, 45, 120, 121, 130])  # 352, 360, 960, 968 and 1040 units: the last two in one and in two parts
 def test_lists_of_every_length(native_libs, batch):
     import torch
     from orinmllm_b200 import capi
@@ -45,7 +45,7 @@ def test_lists_of_every_length(native_libs, batch):
     assert torch.isfinite(together).all() and torch.equal(together, alone)
 
 
-@pytest.mark.parametrize("batch", [20, 100])
+@pytest.mark.parametrize("batch", [20, 100, 140])  # lists in parameters of both sizes, and in the work area
 def test_a_captured_call_carries_its_list(native_libs, batch):
     import torch
     from orinmllm_b200 import capi
