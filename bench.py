@@ -425,7 +425,7 @@ def extra_append(torch, capi):
     return {"workload": "131072 tokens, 8 KV heads x 128, fp16, block 16, random block placement",
             "kernel": "append_token_kernel", "gbs": round(b_plain / t_plain / 1e6, 1),
             "frac": round(b_plain / t_plain / 1e6 / peak, 4), "us": round(t_plain * 1e3, 1), "bytes": b_plain,
-            "rope_append": {"kernel": "rope_append_kernel", "gbs": round(b_rope / t_rope / 1e6, 1),
+            "rope_append": {"kernel": "rope_rows_kernel", "gbs": round(b_rope / t_rope / 1e6, 1),
                             "frac": round(b_rope / t_rope / 1e6 / peak, 4), "us": round(t_rope * 1e3, 1),
                             "bytes": b_rope},
             "peak": peak, "peak_source": src}
