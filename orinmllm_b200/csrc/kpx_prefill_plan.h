@@ -113,8 +113,13 @@ inline void cut_unit(const Unit& d, int k, int& slot, std::vector<Unit>& units, 
   }
 }
 
-// A part costs its rows written and read in fp32, and the call a second launch: together about so many tiles.
-constexpr int kMergeCost = 4;
+// What a cut costs, in tiles: a second launch, the parts' rows written and read in fp32, and the clock, which rises
+// where a last round leaves clusters idle and no longer does when they share its work.  Fitted to calls cut and whole
+// (us, parts, tiles of the fullest cluster): 28/4 heads, 4 x 512 tokens behind 1536 79.7 / 70.5 (72, 52 / 61); 32/8, 20 x
+// 64 behind 1500 51.9 / 53.9 (72, 32 / 42); 8/8, 10 x 128 behind 1000 25.4 / 27.5 (48, 13 / 20); 32/8, 448 behind 6000
+// 65.7 / 60.0 (280, 44 / 52); 64/8, 512 behind 16384 301 / 307 (216, 233 / 263); 8/8, 16 x 128 behind 8192 164.4 / 162.2
+// (216, 118 / 132).
+constexpr int cut_cost(int64_t parts, int64_t load) { return int(4 + parts / 24 + load / 20); }
 
 // The work list of whole units (a cluster can take any number of them).  split: -1 cut where it pays, 0 never, 2..4
 // always, into that many parts (tests).
@@ -138,18 +143,24 @@ inline WorkList plan_units(std::vector<Unit> units, int clusters, int split) {
   // Cut along the keys where whole units leave many clusters idle for long.
   const int64_t even = (tiles + int64_t(n) * kUnitCost + clusters - 1) / clusters;
   const int idle = load - int(even);
-  if (split == 0 || idle <= kMergeCost || idle * int64_t(8) <= even) return w;
+  if (split == 0 || idle <= cut_cost(0, 0) || idle * int64_t(8) <= even) return w;
   const std::vector<Unit> whole = w.units;
   const std::vector<int32_t> by_length = longest_first(whole);
   // The rules below go by means.  Each gives the best cut that has a slot for every part and, where a finer one would
   // be better, that one with the longest units cut first; what is kept is what the dealing bears out.  (Chosen as if
-  // slots had no end, the longest units stayed whole: 512 tokens, 28/4 heads behind 7168 tokens 105 us against 85
-  // uncut, 32/8 behind 10752 169 against 138, behind 16384 169 against 158.)
+  // slots had no end, the longest units stayed whole and the cut was for nothing: 512 tokens, 28/4 heads behind 7168
+  // tokens 86 us against 67 uncut, 32/8 behind 10752 119 against 104, behind 32768 335 against 308.)
+  auto parts_of = [](const WorkList& cut) {
+    int64_t n = 0;
+    for (const Merge& m : cut.merges) n += m.parts;
+    return n;
+  };
   auto keep_if_shorter = [&](WorkList&& cut) {
     if (cut.merges.empty()) return;
-    const int with_merge = deal_units(cut.units, clusters, cut.order, cut.start) + kMergeCost;
-    if (with_merge >= load) return;
-    load = with_merge;
+    const int of_parts = deal_units(cut.units, clusters, cut.order, cut.start);
+    const int with_cut = of_parts + cut_cost(parts_of(cut), of_parts);
+    if (with_cut >= load) return;
+    load = with_cut;
     w = std::move(cut);
   };
   if (longest > even) {
@@ -167,7 +178,8 @@ inline WorkList plan_units(std::vector<Unit> units, int clusters, int split) {
         cuts += parts > 1;
       }
       const int64_t rounds = (count + clusters - 1) / clusters, mean = (tiles + count * kUnitCost + count - 1) / count;
-      const int cost = int(std::max<int64_t>(c + kUnitCost, rounds * mean)) + kMergeCost;
+      const int64_t of_parts = std::max<int64_t>(c + kUnitCost, rounds * mean);
+      const int cost = int(of_parts) + cut_cost(std::min<int64_t>(slots, kMaxPartSlots), of_parts);
       if (cost < best) {
         best = cost;
         cap = c;
@@ -189,11 +201,12 @@ inline WorkList plan_units(std::vector<Unit> units, int clusters, int split) {
     if (cap > 0 && cap != cap_slots) keep_if_shorter(cut_to(cap));
   } else {  // many units of like length and a thin last round: the shortest, a round's remainder, are cut
     const int rest = n % clusters;
-    const int t = whole[size_t(by_length[size_t(n - 1)])].tile1 + 1;
+    const int t = whole[size_t(by_length[size_t(n - 1)])].tile1 + 1, before = load - t;
     int k = 1, best = (t + kUnitCost) * 8, k_slots = 1;  // eighths of a tile
     for (int c = 2; c <= kMaxParts && rest > 0; ++c) {
       const int rounds = (rest * c + clusters - 1) / clusters;
-      const int cost = rounds * (t * 8 / c + 8 * kUnitCost) + 8 * kMergeCost;
+      const int of_parts = rounds * (t * 8 / c + 8 * kUnitCost);
+      const int cost = of_parts + 8 * cut_cost(std::min(rest * c, kMaxPartSlots), before + of_parts / 8);
       if (cost < best) {
         best = cost;
         k = c;

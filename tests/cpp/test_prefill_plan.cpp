@@ -1,5 +1,5 @@
 // The work list of tensor-core prefill calls: every unit's keys are there once, parts have a slot each, and a call is
-// cut only where that shortens its fullest cluster by more than the merge costs.
+// cut only where that shortens its fullest cluster by more than the cut costs.
 #include <cstdio>
 #include <set>
 
@@ -73,10 +73,12 @@ static void check(const Call& call, int clusters, int split) {
   }
   EXPECT(parts == 0);
 
+  int cut_parts = 0;
+  for (const Merge& m : w.merges) cut_parts += m.parts;
   if (split < 0) {
     const int before = fullest(uncut, clusters), after = fullest(w, clusters);
     if (w.merges.empty()) EXPECT(w.units.size() == whole.size() && after == before);
-    else EXPECT(after + kMergeCost < before);
+    else EXPECT(after + cut_cost(cut_parts, after) < before);
   }
 }
 
