@@ -28,21 +28,21 @@ constexpr int64_t kRowsFrom = 400, kRowsPairs = 1400;
 // brings anyway: bf16 28/4, 1 and 64 tokens 1.89 / 2.14 us early, 1.81 / 2.06 flat) and cost registers: an SM holds
 // fewer CTAs (16-bit rows 3 for 5, fp32 4 for 6).  So that form is for calls that it holds at once, and beyond what the
 // other holds at once for those that it takes one round more for at most; heads wider than 128 gain more by it and
-// take it there in any case.  A sixteenth more than it holds at once costs next to
-// nothing.
+// take it in any case.  A sixteenth of a round more costs next to nothing
+// (heads of 64, 32/8, 2048 tokens, 1792 CTAs, four early rounds and 16 CTAs: 8.0 us early, 8.5 flat, alone).
 // norm + RoPE + append and a decode launch of 64 short sequences, us, flat / early: fp16 32/8 heads of 128, 256 tokens
 // (448 CTAs) 15.3 / 14.6, 320 (560) 15.4 / 15.9; 64/8, 256 (704) 16.2 / 16.7, 320 (880) 18.4 / 16.7; heads of 64, 32/8,
 // 800 (700) 14.8 / 15.5, 1600 (1400) 17.3 / 18.4; fp32 32/8, 160 (560) 15.0 / 13.9, 224 (784) 15.1 / 15.6, 320 (1120)
-// 17.1 / 15.8; heads of 256, bf16 28/4, 900 (2250) 26.0 / 21.8, 8000 151 / 116, fp32 32/8, 8000 213 / 206.
+// 17.1 / 15.8; heads of 256, bf16 28/4, 256 (640) 14.5 / 14.3, 900 (2250) 26.0 / 21.8, 8000 151 / 116, fp16 12/2, 600 (675) 11.7 /
+// 11.9, fp32 32/8, 8000 213 / 206.
 inline RopeForm rope_form(const RopeCall& c) {
   if (c.elt_bytes == 2 && c.head_size == 128 && c.tokens >= kRowsFrom)
     return c.tokens < kRowsPairs ? RopeForm::kOneToken : RopeForm::kTwoTokens;
   if (!c.norm || !c.aligned) return RopeForm::kFlat;
-  auto at_once = [&](int64_t fit) { return c.ctas <= fit + fit / 16; };
-  auto rounds = [&](int64_t fit) { return (c.ctas + fit - 1) / fit; };
-  if (at_once(c.early_fit)) return RopeForm::kEarlyTables;
-  if (at_once(c.flat_fit)) return RopeForm::kFlat;
-  return c.head_size > 128 || rounds(c.early_fit) <= rounds(c.flat_fit) + 1 ? RopeForm::kEarlyTables : RopeForm::kFlat;
+  auto rounds = [&](int64_t fit) { return (c.ctas + fit - 1 - fit / 16) / fit; };
+  const int64_t early = rounds(c.early_fit), flat = rounds(c.flat_fit);
+  if (early <= 1 || c.head_size > 128) return RopeForm::kEarlyTables;
+  return flat > 1 && early <= flat + 1 ? RopeForm::kEarlyTables : RopeForm::kFlat;
 }
 
 }  // namespace kpx

@@ -30,13 +30,13 @@ int main() {
   for (int n : {1400, 131072}) expect(two, 2, 128, 12, 2, n, false);
   // heads of 64: two rounds more than the flat form are too many
   for (int n : {600, 800, 1600}) expect(flat, 2, 64, 32, 8, n);
-  for (int n : {1, 400}) expect(early, 2, 64, 32, 8, n);
+  for (int n : {1, 400, 1200, 2048}) expect(early, 2, 64, 32, 8, n);
   // fp32: never the form of a CTA per token
   for (int n : {1, 64, 160, 288, 399, 800}) expect(early, 4, 128, 32, 8, n);
   for (int n : {192, 224, 256, 20000}) expect(flat, 4, 128, 32, 8, n);
-  // heads of 256: early beyond the flat form's first round
-  for (int n : {1, 399, 900, 8000}) expect(early, 2, 256, 28, 4, n);
-  expect(flat, 2, 256, 12, 2, 600);
+  // heads of 256: early whatever the size
+  for (int n : {1, 200, 399, 900, 8000}) expect(early, 2, 256, 28, 4, n);
+  expect(early, 4, 256, 12, 2, 399);
   // no norm, or tables off 16-byte boundaries
   for (int n : {1, 256, 399}) expect(flat, 2, 128, 32, 8, n, false), expect(flat, 2, 128, 32, 8, n, true, false), expect(flat, 4, 128, 32, 8, n, false);
   return bad != 0;
